@@ -686,11 +686,8 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
     }
     // FP32 batches of small GEMMs (M, N <= 64; tensor-core tiles would be mostly
     // padding with a few k-steps each): plain FP32 on CUDA cores
-    if (dt == OME_F32 && M <= 64 && N <= 64 && L >= 8) {
-      trace_path("  -> simt 64x64");
-      return cuda_err(launch_gemm_simt_small_f32(g, s), "simt small gemm");
-    }
-    if (dt == OME_F32 && prec != OME_PREC_FP32 && gemm_split_supported(g)) {
+    const bool small_batch = dt == OME_F32 && M <= 64 && N <= 64 && L >= 8;
+    if (dt == OME_F32 && prec != OME_PREC_FP32 && !small_batch && gemm_split_supported(g)) {
       // output mode groups of several modes: C offset tables for the epilogues
       // (filled by the packed GEMM's pack launch, else by their own kernel)
       int64_t* tab = nullptr;
