@@ -696,6 +696,24 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       void* w = avail ? ctx->ws + ((ctx->ws_top + 255) & ~(size_t)255) : nullptr;
       const int nterms = prec == OME_PREC_BF16X3 ? 2 : 3;
       const int choice = gemm_kernel_choice(g);
+      // Small products on the FP64 matrix instructions: below 2^25 multiply-adds
+      // the tensor-core kernel's fixed 11-25 us (two operands' splits, eight
+      // k-steps of accumulators) exceed the whole product here (64 x 16 x 8
+      // 10.6 -> 5.8 us, 256^3 24.4 -> 12.3, 512 x 512 x 128 17.7 -> 12.3; above,
+      // 1024 x 1024 x 64 13.9 against 19.6), and sums in Float64 are the more
+      // exact.  Where an operand's K runs over several modes and is not
+      // contiguous, its converters evaluate a mixed-radix offset per element and
+      // the line lies eight times higher (1024 x 512 x 512 in three K modes 143
+      // against 48 us).
+      const double macs = (double)M * (double)N * (double)K * (double)L;
+      const bool k_scattered =
+          g.nk > 1 && (g.k_ext[0] % 8 != 0 || g.k_sa[0] != 1 || g.k_sb[0] != 1);
+      if (choice == 0 && macs <= (k_scattered ? 0x1p28 : 0x1p25)) {
+        trace_path("  -> small");
+        cudaError_t e = launch_gemm_small_f32(g, w, avail, ctx->num_sms, s);
+        if (e != cudaErrorNotSupported) return cuda_err(e, "small gemm");
+        cudaGetLastError();
+      }
       if (choice == 2) {
         cudaError_t e = launch_gemm_tma2(g, nterms, w, avail, ctx->num_sms, s);
         if (e != cudaErrorNotSupported) {

@@ -7,6 +7,7 @@
 // FP32 comparison path.  Operands are read in place through per-group mode
 // strides, so no permuted copy is ever materialised; the output permutation
 // is absorbed in the epilogue's strides.
+#include <cooperative_groups.h>
 #include <string.h>
 #include <algorithm>
 #include "kernels.h"
@@ -34,7 +35,8 @@ struct SimtArgs {
   int32_t S;                       // K splits (1: the epilogue writes C)
   int64_t kchunk;                  // K per split
   int64_t tiles_m, tiles_n, units;
-  void* partial;                   // S > 1: [S][L][M][N]
+  int32_t cluster;                 // 1: a tile's splits form a cluster and add up in shared memory
+  void* partial;                   // S > 1 without a cluster: [S][L][M][N]
   int64_t p_elems;                 // its capacity in elements (self-check)
   Scalar sx, sy;
   int sy_zero, sx_one;
@@ -159,7 +161,52 @@ struct SimtTile {
   static constexpr size_t TABLES = (2 * BM + 2 * BN + (STAGES + 1) * 2 * BK) * sizeof(int64_t);
   static constexpr size_t SMEM = TABLES + (size_t)STAGES * STAGE * sizeof(T) +
                                  (std::is_same<T, long long>::value ? 2 * (BM + BN) * BK : 0);
+  static constexpr bool CLUSTER = BM * BN <= STAGES * STAGE;   // a tile fits the stages
 };
+
+// Unit u -> tile, K split and batch; a cluster's blocks are a tile's splits.
+__device__ __forceinline__ void simt_unit(const SimtArgs& g, int64_t u, int64_t& tm, int64_t& tn, int64_t& spi,
+                                          int64_t& l) {
+  int64_t r = u;
+  if (g.cluster) {
+    spi = r % g.S;
+    r /= g.S;
+  }
+  tm = r % g.tiles_m;
+  r /= g.tiles_m;
+  tn = r % g.tiles_n;
+  r /= g.tiles_n;
+  if (!g.cluster) {
+    spi = r % g.S;
+    r /= g.S;
+  }
+  l = r;
+}
+
+// A tile's partial sums, one per block of the cluster in `tile` ([BM][BN],
+// type V), added in split order; each block finishes its share of the tile.
+template <class A, class V, int BM, int BN, int NT>
+__device__ __forceinline__ void simt_cluster_finish(const SimtArgs& g, V* tile, const int64_t* cm, const int64_t* cn,
+                                                    int64_t lc, int64_t m0, int64_t n0, int rank, int tid) {
+  using T = typename A::T;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();
+  const T sx = scalar_as<T>(g.sx), sy = scalar_as<T>(g.sy);
+  T* Cp = static_cast<T*>(g.C);
+  for (int e = rank * NT + tid; e < BM * BN; e += g.S * NT) {
+    const int mi = e / BN, nj = e % BN;
+    if (m0 + mi >= g.M || n0 + nj >= g.N) continue;
+    V acc = *cl.map_shared_rank(tile + e, 0);
+    for (int q = 1; q < g.S; ++q) {
+      const V w = *cl.map_shared_rank(tile + e, q);
+      if constexpr (std::is_same<V, T>::value) acc = A::add(acc, w);
+      else acc = acc + w;
+    }
+    T* cp = Cp + lc + cm[mi] + cn[nj];
+    *cp = epilogue<A>((T)acc, cp, sx, sy, g.sy_zero, g.sx_one);
+  }
+  cl.sync();   // the other blocks have read this one's sums
+}
 
 // One operand of a tile: where its rows and its split's k start.
 template <class T>
@@ -294,12 +341,8 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_simt(const __grid_const
   griddep_launch_dependents();
 
   for (int64_t u = blockIdx.x; u < g.units; u += gridDim.x) {
-    int64_t r = u;
-    const int64_t tm = r % g.tiles_m;
-    r /= g.tiles_m;
-    const int64_t tn = r % g.tiles_n;
-    r /= g.tiles_n;
-    const int64_t spi = r % g.S, l = r / g.S;
+    int64_t tm, tn, spi, l;
+    simt_unit(g, u, tm, tn, spi, l);
     const int64_t m0 = tm * BM, n0 = tn * BN;
     const int64_t kbeg = spi * g.kchunk;
     const int64_t kend = min(g.K, kbeg + g.kchunk);
@@ -430,6 +473,16 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_simt(const __grid_const
     cp_wait<0>();
     if constexpr (I64) flush();
     const int64_t lc = simt_off(l, g.l, g.l_sc, g.wide);
+    if (g.cluster) {
+      __syncthreads();   // the stages are free
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+          sm[(ty * TM + i) * BN + (j / G) * TX * G + tx * G + j % G] = Mac::value(acc[i][j]);
+      simt_cluster_finish<A, T, BM, BN, NT>(g, sm, cm, cn, lc, m0, n0, (int)spi, tid);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       const int64_t m = m0 + ty * TM + i;
@@ -523,39 +576,73 @@ struct SimtChoice {
   double clocks = 1e300;
   int cfg = 0;
   int64_t S = 1;
+  bool cluster = false;
 };
 
 template <class A, class C>
-static void simt_consider(SimtChoice& best, int cfg, double eff, int occ, const SimtArgs& g, int num_sms,
+static void simt_consider(SimtChoice& best, int cfg, double eff, int occ, double lat, const SimtArgs& g, int num_sms,
                           size_t ws_bytes) {
   const double tiles = (double)((g.M + C::BM - 1) / C::BM) * (double)((g.N + C::BN - 1) / C::BN) * (double)g.L;
   const double es = sizeof(typename A::T);
-  const int64_t smax = std::min<int64_t>(128, std::max<int64_t>(1, g.K / 64));
-  for (int64_t S = 1; S <= smax; S += S < 16 ? 1 : S / 8) {
-    const double out = (double)g.M * (double)g.N * (double)g.L;
-    if (S > 1 && (double)S * out * es > (double)ws_bytes) break;
+  const double out = (double)g.M * (double)g.N * (double)g.L;
+  auto estimate = [&](int64_t S) {
     const int64_t kc = ((g.K + S - 1) / S + C::BK - 1) / C::BK * C::BK;
     const double units = tiles * (double)((g.K + kc - 1) / kc);
     const double per_sm = std::ceil(units / num_sms), rounds = std::ceil(units / ((double)num_sms * occ));
     // an SM with fewer resident blocks than `occ` does not reach the rate
     const double fill = std::min(1.0, 0.6 + 0.4 * std::min(per_sm, (double)occ) / occ);
-    double clk = per_sm * (double)kc * C::BM * C::BN / (SimtRate<A>::v * eff * fill) + rounds * 4000.0 +
-                 out * es / 3500.0;
-    if (S > 1) clk += 6000.0 + 2.0 * S * out * es / 3500.0;
-    if (clk < best.clocks) best = SimtChoice{clk, cfg, S};
+    // a block's stages follow each other at no less than their latency (`lat`
+    // clocks per k: the FP64 matrix instructions' dependent sums are the slower)
+    const double work = per_sm * (double)kc * C::BM * C::BN / (SimtRate<A>::v * eff * fill);
+    return std::max(work, rounds * (double)kc * lat) + rounds * 4000.0 + out * es / 3500.0;
+  };
+  const int64_t smax = std::min<int64_t>(128, std::max<int64_t>(1, g.K / 64));
+  for (int64_t S = 1; S <= smax; S += S < 16 ? 1 : S / 8) {
+    if (S > 1 && (double)S * out * es > (double)ws_bytes) break;
+    const double clk = estimate(S) + (S > 1 ? 7000.0 + 2.0 * S * out * es / 3500.0 : 0.0);
+    if (clk < best.clocks) best = SimtChoice{clk, cfg, S, false};
   }
+  // two to eight splits as a cluster: no second launch, no partials in memory
+  // (16 x 16 x 256 11.9 -> 7.1 us); with more than two blocks per SM the
+  // clusters' placement costs more than that (300^3 in 8 splits 25 us, in 2 16)
+  if (C::CLUSTER)
+    for (int64_t S = 2; S <= 8 && S * C::BK <= g.K && tiles * S <= 2.0 * num_sms; S *= 2) {
+      const double clk = estimate(S) + 2000.0;
+      if (clk < best.clocks) best = SimtChoice{clk, cfg, S, true};
+    }
 }
 
 // Tile counts and K split of a chosen configuration.
 template <class C>
-static void simt_plan(SimtArgs& g, int64_t S, void* workspace) {
+static void simt_plan(SimtArgs& g, const SimtChoice& ch, void* workspace) {
+  const int64_t S = ch.S;
+  g.cluster = ch.cluster;
   g.tiles_m = (g.M + C::BM - 1) / C::BM;
   g.tiles_n = (g.N + C::BN - 1) / C::BN;
   g.kchunk = S > 1 ? ((g.K + S - 1) / S + C::BK - 1) / C::BK * C::BK : g.K;
-  g.S = (int32_t)(S > 1 ? (g.K + g.kchunk - 1) / g.kchunk : 1);
+  // (a cluster keeps its size; its last splits may be empty)
+  g.S = (int32_t)(ch.cluster ? S : S > 1 ? (g.K + g.kchunk - 1) / g.kchunk : 1);
   g.units = g.tiles_m * g.tiles_n * g.S * g.L;
   g.partial = workspace;
   g.p_elems = (int64_t)g.S * g.L * g.M * g.N;
+}
+
+template <class K>
+static cudaError_t launch_simt_kernel(K* kernel, const SimtArgs& g, int threads, size_t smem, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<int64_t>(g.units, 0x7fffffff));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)g.S;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = g.cluster ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, g);
+  count_launch();
+  return e;
 }
 
 template <class A>
@@ -570,36 +657,51 @@ static cudaError_t launch_simt_finish(const SimtArgs& g, int num_sms, cudaStream
 }
 
 template <class A, class C>
-static cudaError_t launch_simt_cfg(SimtArgs& g, int64_t S, void* workspace, int num_sms, cudaStream_t s) {
-  simt_plan<C>(g, S, workspace);
+static cudaError_t launch_simt_cfg(SimtArgs& g, const SimtChoice& ch, void* workspace, int num_sms, cudaStream_t s) {
+  simt_plan<C>(g, ch, workspace);
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(attr, k_gemm_simt<A, C>, (int)C::SMEM);
   if (e != cudaSuccess) return e;
-  const unsigned grid = (unsigned)std::min<int64_t>(g.units, 0x7fffffff);
   {
     KernelTimer kt(s, "k_gemm_simt");
-    k_gemm_simt<A, C><<<grid, C::NT, C::SMEM, s>>>(g);
+    e = launch_simt_kernel(k_gemm_simt<A, C>, g, C::NT, C::SMEM, s);
   }
-  count_launch();
-  e = cudaGetLastError();
-  return e != cudaSuccess || g.S == 1 ? e : launch_simt_finish<A>(g, num_sms, s);
+  return e != cudaSuccess || g.S == 1 || g.cluster ? e : launch_simt_finish<A>(g, num_sms, s);
 }
 
 // ---------------------------------------------------------------------------
 // FP64 matrix instructions
 // ---------------------------------------------------------------------------
 
-// Tile configuration of k_gemm_dmma: WM x WN per warp.
-template <class T, int BM_, int BN_, int WM_, int WN_, int BK_, int STAGES_, int MINB_>
+// Tile configuration of k_gemm_dmma: WM x WN per warp; elements of type T are
+// multiplied as W (double, or complex double).  With T = W the fragments are
+// read from the stages; otherwise a stage is widened into one of two buffers.
+template <class T, class W_, int BM_, int BN_, int WM_, int WN_, int BK_, int STAGES_, int MINB_>
 struct DmmaTile {
+  using W = W_;
+  static constexpr bool WIDEN = !std::is_same<T, W>::value;
   static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, BK = BK_, STAGES = STAGES_, MINB = MINB_;
   static constexpr int NT = (BM / WM) * (BN / WN) * 32;
-  static constexpr int PAD = 32 / (int)sizeof(T);     // fragment reads are conflict-free
+  static constexpr int PAD = 32 / (int)sizeof(W);     // fragment reads are conflict-free
   static constexpr int PA = BM + PAD, PB = BN + PAD;
   static constexpr int STAGE = (PA + PB) * BK;
   static constexpr size_t TABLES = (2 * BM + 2 * BN + (STAGES + 1) * 2 * BK) * sizeof(int64_t);
-  static constexpr size_t SMEM = TABLES + (size_t)STAGES * STAGE * sizeof(T);
+  static constexpr size_t SMEM = TABLES + (size_t)STAGES * STAGE * sizeof(T) +
+                                 (WIDEN ? 2 * (size_t)STAGE * sizeof(W) : 0);
+  static constexpr bool CLUSTER = BM * BN * sizeof(W) <= SMEM - TABLES;   // a tile fits the stages
 };
+
+// The elements that this thread brought into a stage, widened to double (its
+// own copies have landed; the same places as simt_load's).
+template <int ROWS, int P, int BK, int NT>
+__device__ __forceinline__ void simt_widen(double* w, const float* st, int rowfast, int tid) {
+#pragma unroll
+  for (int r = 0; r < ROWS * BK / NT; ++r) {
+    const int row = rowfast ? tid % ROWS : tid / BK + r * (NT / BK);
+    const int k = rowfast ? tid / ROWS + r * (NT / ROWS) : tid % BK;
+    w[k * P + row] = (double)st[k * P + row];
+  }
+}
 
 // D += A B on a 16 x 4 by 4 x 8 block: lane (g, t) = (lane / 4, lane % 4) holds
 // A(g, t), A(g + 8, t), B(t, g) and D(g, 2t), D(g, 2t + 1), D(g + 8, 2t), D(g + 8, 2t + 1).
@@ -619,7 +721,8 @@ __device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[2], doubl
 template <class A, class C>
 __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_constant__ SimtArgs g) {
   using T = typename A::T;
-  constexpr bool CPLX = sizeof(T) == 16;
+  using W = typename C::W;
+  constexpr bool CPLX = sizeof(W) == 16;
   constexpr int P = CPLX ? 2 : 1;                   // real accumulators per output
   constexpr int BM = C::BM, BN = C::BN, BK = C::BK, NT = C::NT, ST = C::STAGES;
   constexpr int PA = C::PA, PB = C::PB, MI = C::WM / 16, NI = C::WN / 8;
@@ -630,6 +733,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
   int64_t* cn = bn + BN;
   int64_t* kt = cn + BN;
   T* sm = reinterpret_cast<T*>(kt + (ST + 1) * 2 * BK);
+  W* wide = reinterpret_cast<W*>(sm + ST * C::STAGE);   // widened stages [2]
   const T* Ap = static_cast<const T*>(g.A);
   const T* Bp = static_cast<const T*>(g.B);
   T* Cp = static_cast<T*>(g.C);
@@ -640,12 +744,8 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
   griddep_launch_dependents();
 
   for (int64_t u = blockIdx.x; u < g.units; u += gridDim.x) {
-    int64_t r = u;
-    const int64_t tm = r % g.tiles_m;
-    r /= g.tiles_m;
-    const int64_t tn = r % g.tiles_n;
-    r /= g.tiles_n;
-    const int64_t spi = r % g.S, l = r / g.S;
+    int64_t tm, tn, spi, l;
+    simt_unit(g, u, tm, tn, spi, l);
     const int64_t m0 = tm * BM, n0 = tn * BN;
     const int64_t kbeg = spi * g.kchunk;
     const int64_t kend = min(g.K, kbeg + g.kchunk);
@@ -695,11 +795,21 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
     for (int s = 0; s < ST - 1; ++s) issue(s);
     for (int it = 0; it < nk; ++it) {
       cp_wait<ST - 2>();
+      const W* ws;
+      if constexpr (C::WIDEN) {
+        W* wd = wide + (it & 1) * C::STAGE;
+        const T* st = sm + (it % ST) * C::STAGE;
+        simt_widen<BM, PA, BK, NT>(wd, st, g.a_rowfast, tid);
+        simt_widen<BN, PB, BK, NT>(wd + PA * BK, st + PA * BK, g.b_rowfast, tid);
+        ws = wd;
+      } else {
+        ws = sm + (it % ST) * C::STAGE;
+      }
       __syncthreads();
       issue(it + ST - 1);
       if (tid < 2 * BK) ktable(it + ST, tid);
-      const T* as = sm + (it % ST) * C::STAGE + tt * PA + wm + gg;
-      const T* bs = sm + (it % ST) * C::STAGE + PA * BK + tt * PB + wn + gg;
+      const W* as = ws + tt * PA + wm + gg;
+      const W* bs = ws + PA * BK + tt * PB + wn + gg;
 #pragma unroll
       for (int kk = 0; kk < BK; kk += 4) {
         if constexpr (!CPLX) {
@@ -750,6 +860,22 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
     }
     cp_wait<0>();
     const int64_t lc = simt_off(l, g.l, g.l_sc, g.wide);
+    if (g.cluster) {
+      __syncthreads();   // the stages are free
+      W* tile = reinterpret_cast<W*>(sm);
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            W& t = tile[(wm + 16 * i + 8 * (q >> 1) + gg) * BN + wn + 8 * j + 2 * tt + (q & 1)];
+            if constexpr (CPLX) t = W{acc[i][j][0][q], acc[i][j][P - 1][q]};
+            else t = acc[i][j][0][q];
+          }
+      simt_cluster_finish<A, W, BM, BN, NT>(g, tile, cm, cn, lc, m0, n0, (int)spi, tid);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -766,7 +892,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
             if (n >= g.N) continue;
             T v;
             if constexpr (CPLX) v = T{acc[i][j][0][2 * h + q], acc[i][j][P - 1][2 * h + q]};
-            else v = acc[i][j][0][2 * h + q];
+            else v = (T)acc[i][j][0][2 * h + q];
             if (g.S > 1) {
               const int64_t po = ((spi * g.L + l) * g.M + m) * g.N + n;
               if (po < g.p_elems) static_cast<T*>(g.partial)[po] = v;
@@ -782,19 +908,16 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_const
 }
 
 template <class A, class C>
-static cudaError_t launch_dmma_cfg(SimtArgs& g, int64_t S, void* workspace, int num_sms, cudaStream_t s) {
-  simt_plan<C>(g, S, workspace);
+static cudaError_t launch_dmma_cfg(SimtArgs& g, const SimtChoice& ch, void* workspace, int num_sms, cudaStream_t s) {
+  simt_plan<C>(g, ch, workspace);
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(attr, k_gemm_dmma<A, C>, (int)C::SMEM);
   if (e != cudaSuccess) return e;
-  const unsigned grid = (unsigned)std::min<int64_t>(g.units, 0x7fffffff);
   {
     KernelTimer kt(s, "k_gemm_dmma");
-    k_gemm_dmma<A, C><<<grid, C::NT, C::SMEM, s>>>(g);
+    e = launch_simt_kernel(k_gemm_dmma<A, C>, g, C::NT, C::SMEM, s);
   }
-  count_launch();
-  e = cudaGetLastError();
-  return e != cudaSuccess || g.S == 1 ? e : launch_simt_finish<A>(g, num_sms, s);
+  return e != cudaSuccess || g.S == 1 || g.cluster ? e : launch_simt_finish<A>(g, num_sms, s);
 }
 
 static void simt_group(SimtGroup& o, int n, const int64_t* ext, const int64_t* s0, const int64_t* s1) {
@@ -806,18 +929,13 @@ static void simt_group(SimtGroup& o, int n, const int64_t* ext, const int64_t* s
   }
 }
 
-// CUDA-core GEMM: tile shape and K split by the estimate above; split
-// partials go to `workspace`.
-template <class A>
-static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, size_t ws_bytes, int num_sms,
-                                         cudaStream_t s) {
-  using T = typename A::T;
-  if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
-  for (int i = 0; i < q.nm; ++i) if (q.m_ext[i] > 0xffffffffll) return cudaErrorNotSupported;
-  for (int i = 0; i < q.nn; ++i) if (q.n_ext[i] > 0xffffffffll) return cudaErrorNotSupported;
-  for (int i = 0; i < q.nk; ++i) if (q.k_ext[i] > 0xffffffffll) return cudaErrorNotSupported;
-  for (int i = 0; i < q.nl; ++i) if (q.l_ext[i] > 0xffffffffll) return cudaErrorNotSupported;
-  SimtArgs g;
+// k_gemm_simt's / k_gemm_dmma's arguments from a contraction; false if an
+// extent does not fit the tables.
+static bool simt_args(SimtArgs& g, const GemmArgs& q) {
+  for (int i = 0; i < q.nm; ++i) if (q.m_ext[i] > 0xffffffffll) return false;
+  for (int i = 0; i < q.nn; ++i) if (q.n_ext[i] > 0xffffffffll) return false;
+  for (int i = 0; i < q.nk; ++i) if (q.k_ext[i] > 0xffffffffll) return false;
+  for (int i = 0; i < q.nl; ++i) if (q.l_ext[i] > 0xffffffffll) return false;
   g.C = q.C;
   g.K = q.K;
   g.L = q.L;
@@ -846,6 +964,18 @@ static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, siz
   g.sy = q.sy;
   g.sy_zero = q.sy_zero;
   g.sx_one = q.sx_one;
+  return true;
+}
+
+// CUDA-core GEMM: tile shape and K split by the estimate above; split
+// partials go to `workspace`.
+template <class A>
+static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, size_t ws_bytes, int num_sms,
+                                         cudaStream_t s) {
+  using T = typename A::T;
+  if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
+  SimtArgs g;
+  if (!simt_args(g, q)) return cudaErrorNotSupported;
   SimtChoice best;
   if constexpr (std::is_same<A, AlgF64>::value || std::is_same<A, AlgC64>::value) {
     // FP64 matrix instructions once both sides fill a few of their tiles: the
@@ -853,30 +983,30 @@ static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, siz
     // 2368 x 2048 x 2048); below, the smaller CUDA-core tiles waste less
     if (g.M >= 128 && g.N >= 128) {
       constexpr bool Z = std::is_same<A, AlgC64>::value;
-      using D1 = DmmaTile<T, 64, 64, 32, 32, Z ? 8 : 16, Z ? 3 : 4, Z ? 2 : 3>;
-      using D2 = DmmaTile<T, 128, 64, Z ? 32 : 64, 32, Z ? 8 : 16, Z ? 3 : 4, Z ? 1 : 2>;
-      simt_consider<A, D1>(best, 1, 0.8, Z ? 2 : 3, g, num_sms, ws_bytes);
-      simt_consider<A, D2>(best, 2, 0.9, 1, g, num_sms, ws_bytes);
-      if (best.cfg == 1) return launch_dmma_cfg<A, D1>(g, best.S, workspace, num_sms, s);
-      if (best.cfg == 2) return launch_dmma_cfg<A, D2>(g, best.S, workspace, num_sms, s);
+      using D1 = DmmaTile<T, T, 64, 64, 32, 32, Z ? 8 : 16, Z ? 3 : 4, Z ? 2 : 3>;
+      using D2 = DmmaTile<T, T, 128, 64, Z ? 32 : 64, 32, Z ? 8 : 16, Z ? 3 : 4, Z ? 1 : 2>;
+      simt_consider<A, D1>(best, 1, 0.8, Z ? 2 : 3, Z ? 500 : 200, g, num_sms, ws_bytes);
+      simt_consider<A, D2>(best, 2, 0.9, 1, Z ? 500 : 300, g, num_sms, ws_bytes);
+      if (best.cfg == 1) return launch_dmma_cfg<A, D1>(g, best, workspace, num_sms, s);
+      if (best.cfg == 2) return launch_dmma_cfg<A, D2>(g, best, workspace, num_sms, s);
     }
   }
   using T1 = SimtTile<T, 32, 32, 4, 2, 16, 4>;
   using T2 = SimtTile<T, 64, 64, 4, 4, 16, sizeof(T) >= 16 ? 1 : 2>;
-  simt_consider<A, T1>(best, 1, 0.35, 8, g, num_sms, ws_bytes);
-  simt_consider<A, T2>(best, 2, 0.7, sizeof(T) >= 16 ? 1 : 2, g, num_sms, ws_bytes);
+  simt_consider<A, T1>(best, 1, 0.35, 8, 40, g, num_sms, ws_bytes);
+  simt_consider<A, T2>(best, 2, 0.7, sizeof(T) >= 16 ? 1 : 2, 40, g, num_sms, ws_bytes);
   if constexpr (sizeof(T) >= 16) {
-    if (best.cfg == 1) return launch_simt_cfg<A, T1>(g, best.S, workspace, num_sms, s);
-    return launch_simt_cfg<A, T2>(g, best.S, workspace, num_sms, s);
+    if (best.cfg == 1) return launch_simt_cfg<A, T1>(g, best, workspace, num_sms, s);
+    return launch_simt_cfg<A, T2>(g, best, workspace, num_sms, s);
   } else {
     // 8 x 8 per thread where the accumulators fit 255 registers (Int64's are 12
     // bytes, the Float64 maximum keeps temporaries)
     constexpr int TN3 = std::is_same<A, AlgI64>::value || std::is_same<A, AlgTF64>::value ? 4 : 8;
     using T3 = SimtTile<T, 128, 16 * TN3, 8, TN3, 8, sizeof(T) <= 4 ? 2 : 1>;
-    simt_consider<A, T3>(best, 3, 0.9, sizeof(T) <= 4 ? 2 : 1, g, num_sms, ws_bytes);
-    if (best.cfg == 1) return launch_simt_cfg<A, T1>(g, best.S, workspace, num_sms, s);
-    if (best.cfg == 2) return launch_simt_cfg<A, T2>(g, best.S, workspace, num_sms, s);
-    return launch_simt_cfg<A, T3>(g, best.S, workspace, num_sms, s);
+    simt_consider<A, T3>(best, 3, 0.9, sizeof(T) <= 4 ? 2 : 1, 80, g, num_sms, ws_bytes);
+    if (best.cfg == 1) return launch_simt_cfg<A, T1>(g, best, workspace, num_sms, s);
+    if (best.cfg == 2) return launch_simt_cfg<A, T2>(g, best, workspace, num_sms, s);
+    return launch_simt_cfg<A, T3>(g, best, workspace, num_sms, s);
   }
 }
 
@@ -1079,6 +1209,19 @@ int simt_bounds_flag() {
     cudaMemcpyToSymbol(g_ome_bounds_simt, &zero, sizeof(int));
   }
   return v;
+}
+
+cudaError_t launch_gemm_small_f32(const GemmArgs& q, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s) {
+  if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
+  SimtArgs g;
+  if (!simt_args(g, q)) return cudaErrorNotSupported;
+  using E1 = DmmaTile<float, double, 32, 32, 16, 16, 32, 3, 4>;
+  using E2 = DmmaTile<float, double, 64, 64, 32, 32, 16, 4, 3>;
+  SimtChoice best;
+  simt_consider<AlgF64, E1>(best, 1, 0.4, 4, 85, g, num_sms, ws_bytes);
+  simt_consider<AlgF64, E2>(best, 2, 0.6, 3, 200, g, num_sms, ws_bytes);
+  if (best.cfg == 1) return launch_dmma_cfg<AlgF32, E1>(g, best, workspace, num_sms, s);
+  return launch_dmma_cfg<AlgF32, E2>(g, best, workspace, num_sms, s);
 }
 
 cudaError_t launch_gemm_simt_ws(ome_dtype dt, const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms,

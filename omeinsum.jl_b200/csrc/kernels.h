@@ -56,6 +56,9 @@ cudaError_t launch_scale(ome_dtype dt, void* y, int nd, const int64_t* ext, cons
 // would leave SMs idle.
 cudaError_t launch_gemm_simt_ws(ome_dtype dt, const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms,
                                 cudaStream_t s);
+// Small FP32 GEMMs: products and sums in Float64 on the FP64 matrix
+// instructions, rounded once at the end (once per split of K).
+cudaError_t launch_gemm_small_f32(const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s);
 // Batched GEMM with the batch mode contiguous in A, B and C and M, N <= 64
 // (4 consecutive batches per CTA staged in shared memory, k_gemm_bstage);
 // cudaErrorNotSupported if the shape differs.

@@ -103,3 +103,28 @@ def test_tropical_f32_special_values(m, k, n):
     got = to_np(got)
     assert got.dtype == np.float32
     assert np.array_equal(got, want.astype(np.float32), equal_nan=True)
+
+
+@pytest.mark.parametrize("code,sizes", [
+    ("ij,jk->ik", dict(i=16, j=8, k=16)),
+    ("ij,jk->ki", dict(i=33, j=31, k=65)),              # one past a tile on each side, K below a stage
+    ("ji,kj->ik", dict(i=16, j=256, k=16)),             # one tile, K split over a cluster
+    ("ij,jk->ik", dict(i=100, j=2000, k=100)),
+    ("ij,jk->ik", dict(i=20, j=30000, k=30)),           # more splits than a cluster holds
+    ("apbqc,xpyqc->abxy", dict(a=5, b=8, x=3, y=7, p=3, q=5, c=4)),    # three k modes
+    ("apbqc,xpyqc->abxy", dict(a=32, b=32, x=16, y=33, p=8, q=8, c=8)),   # above 2^25 products
+])
+def test_small_f32_sums_in_double(code, sizes):
+    """Small FP32 products are summed in Float64 and rounded once (once per
+    split of K beyond a cluster, then their sum): norm-wise below 2e-7."""
+    rng = np.random.default_rng(11)
+    ixs, iy = parse(code)
+    xs = [gen(rng, [sizes[l] for l in ix], "f32") for ix in ixs]
+    want = oracle(ixs, iy, xs, sizes, "f32", wide=True)
+    c = ome.EinCode(ixs, iy)
+    assert_match(to_np(ome.einsum(c, [to_dev(x, "f32") for x in xs], sizes)), want, "f32", 2e-7)
+    y0 = gen(rng, [sizes[l] for l in iy], "f32")
+    yd = to_dev(y0, "f32")
+    ome.einsum_(c, [to_dev(x, "f32") for x in xs], yd, 2, 3, sizes)
+    ome.device_status()
+    assert_match(to_np(yd), 2 * want + 3 * y0.astype(np.float64), "f32", 3e-7)
