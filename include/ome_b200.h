@@ -198,6 +198,13 @@ OME_API int ome_plan_execute(ome_ctx* ctx, ome_plan* plan, void* stream,
                      const void* const* inputs, void* y, const void* sx,
                      const void* sy);
 
+/* The same with strided inputs: in_strides holds every input's element strides
+ * one input after the other, each in the order of its labels (NULL: the inputs
+ * are column-major contiguous). */
+OME_API int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* plan, void* stream,
+                                     const void* const* inputs, const int64_t* in_strides,
+                                     void* y, const void* sx, const void* sy);
+
 /* Slice sharding (the slice loop of src/slicing.jl:118-137 split over ranks;
  * replaces the host-staged examples/slicing_multigpu.jl:54-75).  The slice
  * index space 0..nslices-1 is CartesianIndices order over the sliced labels,
@@ -232,6 +239,12 @@ OME_API int ome_plan_finish(ome_ctx* ctx, ome_plan* plan, void* stream, const vo
 OME_API int ome_plan_gradient(ome_ctx* ctx, ome_plan* plan, void* stream,
                       const void* const* inputs, const void* dy, void* y,
                       void* const* dxs);
+
+/* The same with strided inputs (as in ome_plan_execute_strided); the gradients
+ * are column-major contiguous. */
+OME_API int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* plan, void* stream,
+                                      const void* const* inputs, const int64_t* in_strides,
+                                      const void* dy, void* y, void* const* dxs);
 
 /* Contraction-order search (host) ------------------------------------------
  *

@@ -27,7 +27,7 @@ EXPORTS = [
     "ome_plan_execute_slices", "ome_plan_finish", "ome_reduce_noalloc", "ome_batch_create", "ome_batch_run",
     "ome_batch_info", "ome_batch_destroy", "ome_batch_graph_create", "ome_graph_launch", "ome_graph_destroy",
     "ome_server_create", "ome_server_submit", "ome_server_poll", "ome_server_stats", "ome_server_clock", "ome_server_destroy",
-    "ome_treesa", "ome_greedy", "ome_slice_greedy",
+    "ome_treesa", "ome_greedy", "ome_slice_greedy", "ome_plan_execute_strided", "ome_plan_gradient_strided",
 ]
 
 JOB_COMPLETED, JOB_FAILED, JOB_REJECTED_MEMORY, JOB_REJECTED_WORK = range(4)
@@ -109,6 +109,8 @@ def load() -> C.CDLL:
         lib.ome_plan_peak_bytes.argtypes = [P, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
         lib.ome_plan_execute.argtypes = [P, P, P, C.POINTER(P), P, P, P]
         lib.ome_plan_gradient.argtypes = [P, P, P, C.POINTER(P), P, P, C.POINTER(P)]
+        lib.ome_plan_execute_strided.argtypes = [P, P, P, C.POINTER(P), i64p, P, P, P]
+        lib.ome_plan_gradient_strided.argtypes = [P, P, P, C.POINTER(P), i64p, P, P, C.POINTER(P)]
         lib.ome_plan_slice_count.argtypes = [P, i64p]
         lib.ome_plan_partial_info.argtypes = [P, C.POINTER(C.c_int), C.POINTER(C.c_size_t), C.POINTER(C.c_int)]
         lib.ome_plan_execute_slices.argtypes = [P, P, P, C.POINTER(P), C.c_int64, C.c_int64, P]

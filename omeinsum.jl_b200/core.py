@@ -76,7 +76,11 @@ class EinCode(AbstractEinsum):
         return EinCode([[m.get(l, l) for l in ix] for ix in self.ixs], [m.get(l, l) for l in self.iy])
 
     def __call__(self, *xs, size_info=None):
-        from .engine import einsum
+        from .engine import einsum, einsum_plain
+        if size_info is None:
+            y = einsum_plain(self, xs)
+            if y is not None:
+                return y
         sd = get_size_dict(self.ixs, xs, size_info)
         return einsum(self, xs, sd)
 
@@ -161,6 +165,11 @@ class NestedEinsum(AbstractEinsum):
 
     def __call__(self, *xs, size_info=None):
         from .engine import einsum
+        if size_info is None:
+            from .plan import tree_plain
+            y = tree_plain(self, xs)
+            if y is not None:
+                return y
         sd = get_size_dict(self.getixsv(), xs, size_info)
         return einsum(self, xs, sd)
 
@@ -197,6 +206,11 @@ class SlicedEinsum(AbstractEinsum):
 
     def __call__(self, *xs, size_info=None):
         from .engine import einsum
+        if size_info is None:
+            from .plan import tree_plain
+            y = tree_plain(self, xs)
+            if y is not None:
+                return y
         sd = get_size_dict(self.getixsv(), xs, size_info)
         return einsum(self, xs, sd)
 

@@ -44,6 +44,7 @@ struct ome_plan {
   int prec;
   int ninputs;
   std::vector<std::vector<int32_t>> in_labels;
+  std::vector<int> in_pos;         // where input t's strides start in a caller's stride list
   std::map<int32_t, int64_t> ext;
   std::vector<int32_t> sliced;
   int64_t nslices = 1;
@@ -202,6 +203,7 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   int pos = 0;
   for (int t = 0; t < ninputs; ++t) {
     std::vector<int32_t> l(input_labels + pos, input_labels + pos + input_nlabels[t]);
+    p->in_pos.push_back(pos);
     pos += input_nlabels[t];
     for (int32_t x : l)
       if (!p->ext.count(x)) {
@@ -383,8 +385,39 @@ int ome_plan_peak_bytes(const ome_plan* plan, size_t* forward_bytes, size_t* gra
 
 namespace {
 
+// The caller's input tensors: data, and element strides of all inputs' modes
+// one after the other (NULL: column-major contiguous).
+struct Leaves {
+  const void* const* data;
+  const int64_t* str;
+};
+
+// View of input t; labels in `drop` are fixed at index `fix` as in make_view.
+HView leaf_view(const ome_plan* p, const Leaves& in, int t, const std::vector<int32_t>& drop,
+                const std::vector<int64_t>& fix) {
+  const auto& labs = p->in_labels[t];
+  if (!in.str) return make_view(p, (char*)in.data[t], labs, drop, fix);
+  const int64_t* str = in.str + p->in_pos[t];
+  HView v;
+  v.nd = 0;
+  int64_t off = 0;
+  for (size_t d = 0; d < labs.size(); ++d) {
+    auto it = std::find(drop.begin(), drop.end(), labs[d]);
+    if (it != drop.end()) {
+      off += fix[it - drop.begin()] * str[d];
+    } else {
+      v.lab[v.nd] = labs[d];
+      v.ext[v.nd] = p->ext.at(labs[d]);
+      v.str[v.nd] = str[d];
+      v.nd++;
+    }
+  }
+  v.data = (char*)in.data[t] + off * (int64_t)p->esize;
+  return v;
+}
+
 // Run one node: inputs from children (workspace or leaf views), output view y.
-int run_node(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int j, const void* const* inputs, bool sliced,
+int run_node(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int j, const Leaves& inputs, bool sliced,
              const std::vector<int64_t>& fix, size_t (*off_of)(const PNode&), const HView& y, const Scalar& sx,
              const Scalar& sy, size_t scratch_base) {
   const PNode& n = p->nodes[j];
@@ -398,8 +431,7 @@ int run_node(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int j, const void* const
     if (r >= 0) {
       xs[a] = make_view(p, ctx->ws + off_of(p->nodes[r]), sliced ? p->nodes[r].iy_s : p->nodes[r].iy, none, nofix);
     } else {
-      const int t = -r - 1;
-      xs[a] = make_view(p, (char*)inputs[t], p->in_labels[t], sliced ? p->sliced : none, sliced ? fix : nofix);
+      xs[a] = leaf_view(p, inputs, -r - 1, sliced ? p->sliced : none, sliced ? fix : nofix);
     }
   }
   ctx->ws_top = scratch_base;
@@ -414,7 +446,7 @@ size_t off_keep_of(const PNode& n) { return n.off_keep; }
 // positions: into the F64/C64 buffer `acc` for acc64 plans (the root goes to
 // the temporary first), else straight into the plan-dtype output `acc` with
 // root scale sx and sy = one (the caller initialised or prescaled it).
-int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const void* const* inputs, int64_t b, int64_t e,
+int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, int64_t b, int64_t e,
                char* acc, const Scalar& sx) {
   const ome_dtype dt = p->dt;
   const Scalar one = scalar_one(dt), zero = scalar_zero(dt);
@@ -463,7 +495,13 @@ extern "C" {
 
 int ome_plan_execute(ome_ctx* ctx, ome_plan* p, void* stream, const void* const* inputs, void* y, const void* sxp,
                      const void* syp) {
-  if (!ctx || !p || !inputs || !y || !sxp || !syp) return set_err(OME_INVALID_ARGUMENT, "NULL argument");
+  return ome_plan_execute_strided(ctx, p, stream, inputs, nullptr, y, sxp, syp);
+}
+
+int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void* const* in_data,
+                             const int64_t* in_strides, void* y, const void* sxp, const void* syp) {
+  if (!ctx || !p || !in_data || !y || !sxp || !syp) return set_err(OME_INVALID_ARGUMENT, "NULL argument");
+  const Leaves inputs{in_data, in_strides};
   if (ctx->ws_bytes < p->fwd_bytes)
     return set_err(OME_OUT_OF_MEMORY, "plan needs %zu workspace bytes, context has %zu", p->fwd_bytes, ctx->ws_bytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -549,7 +587,7 @@ int ome_plan_execute_slices(ome_ctx* ctx, ome_plan* p, void* stream, const void*
                       "fill");
     if (rc) return rc;
   }
-  return run_slices(ctx, p, s, inputs, slice_begin, slice_end, (char*)partial, scalar_one(p->dt));
+  return run_slices(ctx, p, s, Leaves{inputs, nullptr}, slice_begin, slice_end, (char*)partial, scalar_one(p->dt));
 }
 
 int ome_plan_finish(ome_ctx* ctx, ome_plan* p, void* stream, const void* partial, void* y, const void* sxp,
@@ -583,7 +621,13 @@ extern "C" {
 
 int ome_plan_gradient(ome_ctx* ctx, ome_plan* p, void* stream, const void* const* inputs, const void* dy, void* y,
                       void* const* dxs) {
-  if (!ctx || !p || !inputs || !y || !dxs) return set_err(OME_INVALID_ARGUMENT, "NULL argument");
+  return ome_plan_gradient_strided(ctx, p, stream, inputs, nullptr, dy, y, dxs);
+}
+
+int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void* const* in_data,
+                              const int64_t* in_strides, const void* dy, void* y, void* const* dxs) {
+  if (!ctx || !p || !in_data || !y || !dxs) return set_err(OME_INVALID_ARGUMENT, "NULL argument");
+  const Leaves inputs{in_data, in_strides};
   if (ctx->ws_bytes < p->grad_bytes)
     return set_err(OME_OUT_OF_MEMORY, "gradient needs %zu workspace bytes, context has %zu", p->grad_bytes,
                    ctx->ws_bytes);
@@ -633,7 +677,7 @@ int ome_plan_gradient(ome_ctx* ctx, ome_plan* p, void* stream, const void* const
         } else if (r >= 0) {
           xs[a] = make_view(p, ctx->ws + p->nodes[r].off_keep, p->nodes[r].iy, none, nofix);
         } else {
-          xs[a] = make_view(p, (char*)inputs[-r - 1], p->in_labels[-r - 1], none, nofix);
+          xs[a] = leaf_view(p, inputs, -r - 1, none, nofix);
         }
       }
       const int r = n.args[i];

@@ -296,6 +296,91 @@ def _run_eincode(ixs, iy, p: _Prepared, y: torch.Tensor, sx, sy, loop_only=False
     return y
 
 
+def plain_layout(xs):
+    """(dtype, device index, [shape, strides, ...]) of CUDA tensors that need no
+    preparation: plain torch tensors of one supported dtype on one device.
+    None for anything else (host arrays, mixed dtypes, lazy conjugates)."""
+    t0 = xs[0]
+    if type(t0) is not torch.Tensor or not t0.is_cuda:
+        return None
+    dt, dev = t0.dtype, t0.get_device()
+    if dt not in _TORCH_TO_OME:
+        return None
+    lay = []
+    for t in xs:
+        if type(t) is not torch.Tensor or t.dtype is not dt or t.get_device() != dev or t.is_conj():
+            return None
+        lay.append(t.shape)
+        lay.append(t.stride())
+    return dt, dev, lay
+
+
+class _FlatCall:
+    """The descriptors of ``code(*xs)`` for one layout of the inputs (per host
+    thread): output shape, C structs and scalars; a call sets the pointers."""
+
+    def __init__(self, code: EinCode, xs, dt, dev):
+        size_dict = get_size_dict(code.ixs, xs)
+        self.shape = tuple(size_dict[l] for l in code.iy)
+        self.strides = _colmajor_strides(self.shape)
+        self.dtype, self.device = dt, torch.device("cuda", dev)
+        self.ome = _TORCH_TO_OME[dt]
+        lm = _LabelMap()
+        self.keep: list = []
+        self.xs = (_lib.Tensor * len(xs))()
+        for i, (ix, t) in enumerate(zip(code.ixs, xs)):
+            self.xs[i] = _tensor_struct(t, [lm(l) for l in ix], self.keep)
+        y = torch.empty_strided(self.shape, self.strides, dtype=dt, device=self.device)
+        self.y = _tensor_struct(y, [lm(l) for l in code.iy], self.keep)
+        self.yref = C.byref(self.y)
+        self.one, self.zero = _scalar_cached(self.ome, True), _scalar_cached(self.ome, False)
+
+
+_FLAT_MAX = 1024
+
+
+def einsum_plain(code: EinCode, xs):
+    """``einsum(code, xs)`` for plain CUDA tensors, without the general path's
+    preparation; None if this call needs that path (it also raises the errors)."""
+    be = get_einsum_backend()
+    if not isinstance(be, B200Backend) or not xs or type(code) is not EinCode:
+        return None
+    lay = plain_layout(xs)
+    if lay is None or len(xs) != len(code.ixs):
+        return None
+    dt, dev, shapes = lay
+    flat = getattr(_TLS, "flat", None)
+    if flat is None:
+        flat = _TLS.flat = {}
+    try:
+        key = (code.iy, *code.ixs, dt, dev, *shapes)
+        call = flat.get(key)
+        if call is None:
+            if dev != _current_device():
+                return None
+            if any(len(ix) != t.dim() for ix, t in zip(code.ixs, xs)) or \
+                    not set(code.iy) <= {l for ix in code.ixs for l in ix}:
+                return None
+            call = _FlatCall(code, xs, dt, dev)
+            if len(flat) >= _FLAT_MAX:
+                flat.pop(next(iter(flat)))
+            flat[key] = call
+    except TypeError:   # unhashable labels
+        return None
+    if dev != _current_device():
+        return None
+    y = torch.empty_strided(call.shape, call.strides, dtype=dt, device=call.device)
+    cx = call.xs
+    for i, t in enumerate(xs):
+        cx[i].data = t.data_ptr()
+    call.y.data = y.data_ptr()
+    rc = _lib.load().ome_einsum(_lib.context(dev).handle, _raw_stream(dev), call.ome, len(xs), cx, call.yref,
+                                call.one, call.zero, be.prec)
+    if rc:
+        check(rc)
+    return y
+
+
 # ----------------------------------------------------------------------------
 # public API
 # ----------------------------------------------------------------------------
@@ -317,6 +402,10 @@ def einsum(code: AbstractEinsum, xs: Sequence[Any], size_dict: Dict[Any, int] | 
         from .plan import run_tree
         return run_tree(code, xs, size_dict)
     if size_dict is None:
+        if not kw:
+            y = einsum_plain(code, xs)
+            if y is not None:
+                return y
         size_dict = get_size_dict(code.getixs(), xs)
     p = _Prepared(xs)
     for l in code.iy:

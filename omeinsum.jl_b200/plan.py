@@ -8,16 +8,17 @@ that runs every node from the device workspace.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from typing import Any, Dict, List, Sequence, Tuple
 
 import torch
 
 from . import _lib
 from ._lib import ArgumentError, check
-from .backends import get_einsum_backend
+from .backends import B200Backend, get_einsum_backend
 from .core import NestedEinsum, SlicedEinsum, get_size_dict
-from .engine import (TropicalTensor, _alloc, _f_contig, _LabelMap, _Prepared, _require_b200, _scalar_buf,
-                     _stream)
+from .engine import (_TLS, _TORCH_TO_OME, TropicalTensor, _alloc, _colmajor_strides, _current_device, _f_contig,
+                     _LabelMap, _Prepared, _raw_stream, _require_b200, _scalar_buf, _stream, plain_layout)
 
 
 class Plan:
@@ -106,6 +107,154 @@ def get_plan(code, size_dict, ome_dtype, prec) -> Plan:
     return p
 
 
+# ----------------------------------------------------------------------------
+# repeated calls: what a tree's evaluation needs besides its data
+# ----------------------------------------------------------------------------
+
+# An input of at most this many elements is read in place whatever its strides;
+# larger ones in another order than column-major are copied once per call, as
+# every slice and every gradient reads them again.
+_IN_PLACE = 4096
+
+
+class _TreeState:
+    """What was seen of a tree object: its nodes with copies of their lists, so
+    that a later call notices any change, and the calls prepared for it."""
+
+    def __init__(self, code):
+        self.sliced = isinstance(code, SlicedEinsum)
+        self.slicing = tuple(code.slicing) if self.sliced else ()
+        self.root = code.eins if self.sliced else code
+        self.nodes = []
+        todo = [self.root]
+        while todo:
+            n = todo.pop()
+            if n.tensorindex < 0:
+                self.nodes.append((n, tuple(n.args), n.eins, tuple(n.eins.ixs), n.eins.iy))
+                todo.extend(n.args)
+            else:
+                self.nodes.append((n, n.tensorindex, None, None, None))
+        self.calls: Dict[Any, "_TreeCall"] = {}
+
+    def holds(self, code) -> bool:
+        if self.sliced and (tuple(code.slicing) != self.slicing or code.eins is not self.root):
+            return False
+        for n, args, eins, ixs, iy in self.nodes:
+            if eins is None:
+                if n.tensorindex != args:
+                    return False
+            elif n.eins is not eins or tuple(n.args) != args or tuple(eins.ixs) != ixs or eins.iy != iy:
+                return False
+        return True
+
+
+class _TreeCall:
+    """A tree evaluated on one layout of plain CUDA inputs (per host thread)."""
+
+    def __init__(self, code, ne, xs, dt, dev, ome, prec, grad):
+        size_dict = get_size_dict(ne.getixsv() if grad else code.getixsv(), xs)
+        self.plan = get_plan(ne if grad else code, size_dict, ome, prec)
+        self.shape = tuple(size_dict[l] for l in ne.eins.iy)
+        self.strides = _colmajor_strides(self.shape)
+        self.device, self.dtype, self.dev = torch.device("cuda", dev), dt, dev
+        self.copied = [i for i, t in enumerate(xs)
+                       if t.numel() > _IN_PLACE and tuple(t.stride()) != _colmajor_strides(t.shape)]
+        self.xlay = [(tuple(t.shape), _colmajor_strides(t.shape)) for t in xs]
+        st = [s for i, t in enumerate(xs) for s in (self.xlay[i][1] if i in self.copied else t.stride())]
+        self.str = (C.c_int64 * max(len(st), 1))(*st)
+        self.one, self.zero = _scalar_buf(ome, True), _scalar_buf(ome, False)
+
+    def prepare(self, xs):
+        """The inputs (kept alive by the caller until the launch returns) and their pointers."""
+        if self.copied:
+            xs = list(xs)
+            for i in self.copied:
+                xs[i] = _f_contig(xs[i])
+        return xs, _ptrs(xs)
+
+
+_STATES_MAX = 128
+
+
+def _tree_call(code, xs, grad):
+    """(call, tropical, raw inputs) of a tree on plain CUDA inputs, or None."""
+    be = get_einsum_backend()
+    if not isinstance(be, B200Backend) or len(xs) == 0 or type(code) not in (NestedEinsum, SlicedEinsum):
+        return None
+    root = code.eins if type(code) is SlicedEinsum else code
+    if type(root) is not NestedEinsum or root.tensorindex >= 0:
+        return None
+    trop = type(xs[0]) is TropicalTensor
+    if trop:
+        if any(type(x) is not TropicalTensor for x in xs):
+            return None
+        xs = [x.data for x in xs]
+    lay = plain_layout(xs)
+    if lay is None:
+        return None
+    dt, dev, shapes = lay
+    if dev != _current_device():
+        return None
+    states = getattr(_TLS, "trees", None)
+    if states is None:
+        states = _TLS.trees = {}
+    held = states.get(id(code))
+    if held is None or held[0]() is not code or not held[1].holds(code):
+        if len(states) >= _STATES_MAX:
+            states.pop(next(iter(states)))
+        held = (weakref.ref(code), _TreeState(code))
+        states[id(code)] = held
+    calls = held[1].calls
+    key = (grad, trop, be.prec, dt, dev, *shapes)
+    call = calls.get(key)
+    if call is None:
+        ome = (_lib.TROP_F32 if dt == torch.float32 else _lib.TROP_F64) if trop else _TORCH_TO_OME[dt]
+        call = _TreeCall(code, root, xs, dt, dev, ome, be.prec, grad)
+        if len(calls) >= 16:
+            calls.pop(next(iter(calls)))
+        calls[key] = call
+    return call, trop, xs
+
+
+def tree_plain(code, xs):
+    """The tree's value for plain CUDA inputs, or None if the call needs the
+    general path (which also raises the errors)."""
+    try:
+        got = _tree_call(code, xs, False)
+    except TypeError:   # unhashable labels
+        return None
+    if got is None:
+        return None
+    call, trop, raw = got
+    raw, ptrs = call.prepare(raw)
+    ctx = _lib.context(call.dev, call.plan.forward_bytes)
+    y = torch.empty_strided(call.shape, call.strides, dtype=call.dtype, device=call.device)
+    check(_lib.load().ome_plan_execute_strided(ctx.handle, call.plan.handle, _raw_stream(call.dev), ptrs, call.str,
+                                               y.data_ptr(), call.one, call.zero))
+    return TropicalTensor(y) if trop else y
+
+
+def gradient_plain(code, xs):
+    """cost_and_gradient of a scalar tree on plain CUDA inputs, or None."""
+    try:
+        got = _tree_call(code, xs, True)
+    except TypeError:
+        return None
+    if got is None or got[0].shape != ():
+        return None
+    call, trop, raw = got
+    raw, ptrs = call.prepare(raw)
+    ctx = _lib.context(call.dev, call.plan.grad_bytes)
+    y = torch.empty_strided(call.shape, call.strides, dtype=call.dtype, device=call.device)
+    new, dt, dev = torch.empty_strided, call.dtype, call.device
+    dxs = [new(sh, st, dtype=dt, device=dev) for sh, st in call.xlay]
+    check(_lib.load().ome_plan_gradient_strided(ctx.handle, call.plan.handle, _raw_stream(call.dev), ptrs, call.str,
+                                                None, y.data_ptr(), _ptrs(dxs)))
+    if trop:
+        return TropicalTensor(y), [TropicalTensor(d) for d in dxs]
+    return y, dxs
+
+
 def _ptrs(ts: Sequence[torch.Tensor]):
     return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
@@ -148,6 +297,10 @@ def tree_gradient(code, xs, dy=None):
     """cost_and_gradient on the device: forward with cached intermediates, then
     einsum_grad per node (src/bp.jl:99-130)."""
     be = _require_b200()
+    if dy is None:
+        got = gradient_plain(code, xs)
+        if got is not None:
+            return got
     ne = code.eins if isinstance(code, SlicedEinsum) else code
     if isinstance(code, NestedEinsum) or isinstance(code, SlicedEinsum):
         pass
