@@ -145,11 +145,6 @@ static void free_batch(ome_batch* b) {
 
 namespace {
 
-int find_lab(const HView& v, int32_t l) {
-  for (int d = 0; d < v.nd; ++d)
-    if (v.lab[d] == l) return d;
-  return -1;
-}
 
 // Reduce one binary einsum to a single-mode-per-group strided GEMM.
 int to_problem(const HView& x1v, const HView& x2v, const HView& yv, GroupProblem& p) {

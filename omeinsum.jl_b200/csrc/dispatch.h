@@ -2,7 +2,9 @@
 // executor: labelled strided views, diagonal (repeated-label) views, label
 // classification and mode sorting/merging.
 #pragma once
+#include <algorithm>
 #include <string>
+#include <vector>
 #include "kernels.h"
 
 struct ome_ctx {
@@ -24,6 +26,70 @@ struct HView {
   int64_t ext[MAXD];
   int64_t str[MAXD];
   int32_t lab[MAXD];
+};
+
+inline int find_lab(const HView& v, int32_t l) {
+  for (int d = 0; d < v.nd; ++d)
+    if (v.lab[d] == l) return d;
+  return -1;
+}
+
+// Mode table: one row per label, one stride column per tensor.
+struct Modes {
+  int n = 0, nt = 0;
+  int64_t ext[2 * MAXD];
+  int64_t str[MAXIN + 1][2 * MAXD];
+
+  void add(int64_t e, const int64_t* s) {
+    ext[n] = e;
+    for (int t = 0; t < nt; ++t) str[t][n] = s[t];
+    n++;
+  }
+  int64_t total() const {
+    int64_t p = 1;
+    for (int i = 0; i < n; ++i) p *= ext[i];
+    return p;
+  }
+  // Drop unit modes; stable sort by |stride of tensor key| (zero strides last);
+  // merge neighbours whose strides are consistent in every tensor.
+  void normalize(int key) {
+    int w = 0;
+    for (int i = 0; i < n; ++i) {
+      if (ext[i] == 1) continue;
+      ext[w] = ext[i];
+      for (int t = 0; t < nt; ++t) str[t][w] = str[t][i];
+      w++;
+    }
+    n = w;
+    std::vector<int> idx(n);
+    for (int i = 0; i < n; ++i) idx[i] = i;
+    auto k = [&](int i) -> uint64_t {
+      int64_t s = str[key][i];
+      if (s == 0) return ~0ull;
+      return (uint64_t)(s < 0 ? -s : s);
+    };
+    std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return k(a) < k(b); });
+    int64_t e2[2 * MAXD], s2[MAXIN + 1][2 * MAXD];
+    for (int i = 0; i < n; ++i) {
+      e2[i] = ext[idx[i]];
+      for (int t = 0; t < nt; ++t) s2[t][i] = str[t][idx[i]];
+    }
+    int m = 0;
+    for (int i = 0; i < n; ++i) {
+      if (m > 0) {
+        bool ok = true;
+        for (int t = 0; t < nt && ok; ++t) ok = s2[t][i] == str[t][m - 1] * ext[m - 1];
+        if (ok) {
+          ext[m - 1] *= e2[i];
+          continue;
+        }
+      }
+      ext[m] = e2[i];
+      for (int t = 0; t < nt; ++t) str[t][m] = s2[t][i];
+      m++;
+    }
+    n = m;
+  }
 };
 
 int set_err(int code, const char* fmt, ...);

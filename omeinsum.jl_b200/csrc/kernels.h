@@ -112,6 +112,33 @@ cudaError_t launch_gemm_bdiag(const GemmArgs& g, int nterms, cudaStream_t s);
 cudaError_t launch_gemm_tma2(const GemmArgs& g, int nterms, void* workspace, size_t ws_bytes, int num_sms,
                              cudaStream_t s);
 
+// A program of small contractions (tiny.cu): nodes sorted by level, every node
+// of a level independent of the others.
+constexpr int TINY_MODES = 16;
+constexpr int64_t TINY_WORK = 1 << 16;   // multiply-adds of one node, at most
+struct TinyMode {
+  int32_t sy, s0, s1;   // strides in the result and the operands
+  uint32_t ext;         // extent (low 24 bits); log2 of it in the high bits, 31 if it is no power of two
+};
+struct TinyNode {
+  const void* x0;
+  const void* x1;       // NULL: one input
+  void* y;
+  uint32_t n_out, n_in;
+  uint32_t item0;       // first warp item of the node in its level
+  uint8_t nout, ninner; // modes [0, nout) are output modes, then the summed ones
+  uint8_t flags;        // TINY_*
+  uint8_t pad;
+  alignas(16) TinyMode mode[TINY_MODES];
+};
+enum TinyFlags { TINY_CONJ0 = 1, TINY_CONJ1 = 2, TINY_CONJY = 4, TINY_WARP = 8 };
+// The node's contraction of labelled views (data pointers are not used); false
+// if it does not fit a TinyNode.
+struct HView;
+bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y);
+// Runs nodes[0..n) (level[i] ascending); one launch per 104 nodes.
+cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, cudaStream_t s);
+
 // Read and clear the CUDA-core GEMM's split-partial self-check flag.
 int simt_bounds_flag();
 // One problem of a grouped launch: C[m,n,l] = sx * sum_k A[m,k,l] B[k,n,l]

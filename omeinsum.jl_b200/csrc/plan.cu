@@ -18,6 +18,8 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "dispatch.h"
@@ -35,6 +37,26 @@ struct PNode {
   size_t off_keep = 0;             // offset of the forward value when all are kept
   size_t off_grad = 0;             // offset of the gradient buffer
   int parent = -1;
+  bool tiny = false;               // (sliced sizes) the node and its whole subtree are small contractions
+  bool tiny_full = false;          // the same with full sizes
+};
+
+// A step of a tiny program: contraction of up to two operands, each a node's
+// value, a node's gradient or an input.
+struct TinyStep {
+  enum Kind { VALUE, GRAD, INPUT, INPUT_GRAD, OUTPUT };
+  int nin = 0, level = 0;
+  Kind kind[3];                    // operands, then the result
+  int ref[3];
+  uint8_t flags = 0;
+};
+
+// Its launch descriptors for one set of input strides.
+struct TinyProgram {
+  std::vector<int64_t> strides;    // the caller's (empty: column-major)
+  bool strided = false, ok = false;
+  std::vector<TinyNode> nodes;
+  std::vector<int> level;
 };
 
 }  // namespace
@@ -55,7 +77,15 @@ struct ome_plan {
   size_t arena_bytes = 0, grad_arena = 0;  // planned buffers (forward / gradient)
   size_t fwd_bytes = 0, grad_bytes = 0;     // plus per-node dispatch scratch
   size_t esize = 0;
+  // steps of the tiny programs, levels ascending: forward on sliced and on
+  // full sizes, reverse sweep; programs built for the last input strides seen
+  // (several threads may evaluate one plan)
+  std::vector<TinyStep> steps[3];
+  std::shared_ptr<const TinyProgram> prog[3];
+  std::mutex prog_mutex;
+  std::vector<std::vector<char>> rev_tiny;   // [node][child]: the gradient step is in the reverse program
 };
+enum { TINY_FWD = 0, TINY_FWD_FULL = 1, TINY_REV = 2 };
 
 namespace {
 
@@ -174,6 +204,129 @@ void canonical_orders(ome_plan* p) {
   }
 }
 
+std::vector<int32_t> drop_sliced(const ome_plan* p, const std::vector<int32_t>& l, bool sliced) {
+  if (!sliced) return l;
+  std::vector<int32_t> r;
+  for (int32_t x : l)
+    if (!contains(p->sliced, x)) r.push_back(x);
+  return r;
+}
+
+// Whether the contraction of operands `xs` into labels `y` is a tiny step:
+// one or two operands, no repeated output label, no label summed in one of
+// two operands only, at most TINY_WORK multiply-adds.
+bool tiny_step(const ome_plan* p, const std::vector<std::vector<int32_t>>& xs, const std::vector<int32_t>& y) {
+  if (xs.empty() || xs.size() > 2) return false;
+  for (size_t i = 0; i < y.size(); ++i)
+    for (size_t k = 0; k < i; ++k)
+      if (y[i] == y[k]) return false;
+  std::vector<int32_t> seen;
+  double work = 1;
+  auto visit = [&](int32_t l) {
+    if (contains(seen, l)) return;
+    seen.push_back(l);
+    work *= (double)p->ext.at(l);
+  };
+  for (int32_t l : y) visit(l);
+  for (size_t i = 0; i < xs.size(); ++i)
+    for (int32_t l : xs[i]) {
+      if (xs.size() == 2 && !contains(y, l) && !contains(xs[1 - i], l) && p->ext.at(l) != 1) return false;
+      visit(l);
+    }
+  return work >= 1 && work <= (double)TINY_WORK;
+}
+
+// The steps that run as tiny programs: forward, the nodes whose whole subtree
+// is tiny; in the reverse sweep, the gradient steps below which all are tiny.
+void plan_tiny(ome_plan* p) {
+  const int nn = (int)p->nodes.size(), root = nn - 1;
+  auto labels = [&](int r, bool sliced) {
+    return drop_sliced(p, r >= 0 ? p->nodes[r].iy : p->in_labels[-r - 1], sliced);
+  };
+  std::vector<int> depth(nn);
+  for (int full = 0; full < 2; ++full) {
+    const bool sliced = !full;
+    std::vector<int> order;
+    for (int j = 0; j < (full || p->sliced.empty() ? nn : root); ++j) {
+      PNode& n = p->nodes[j];
+      bool t = true;
+      int d = 0;
+      std::vector<std::vector<int32_t>> xs;
+      for (int r : n.args) {
+        if (r >= 0) {
+          t = t && (full ? p->nodes[r].tiny_full : p->nodes[r].tiny);
+          d = std::max(d, depth[r] + 1);
+        }
+        xs.push_back(labels(r, sliced));
+      }
+      t = t && tiny_step(p, xs, labels(j, sliced));
+      (full ? n.tiny_full : n.tiny) = t;
+      depth[j] = d;
+      if (t) order.push_back(j);
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return depth[a] < depth[b]; });
+    for (int j : order) {
+      TinyStep s;
+      const PNode& n = p->nodes[j];
+      s.nin = (int)n.args.size();
+      s.level = depth[j];
+      for (int a = 0; a < s.nin; ++a) {
+        s.kind[a] = n.args[a] >= 0 ? TinyStep::VALUE : TinyStep::INPUT;
+        s.ref[a] = n.args[a] >= 0 ? n.args[a] : -n.args[a] - 1;
+      }
+      s.kind[2] = j == root ? TinyStep::OUTPUT : TinyStep::VALUE;   // (the root last: all others are below it)
+      s.ref[2] = j;
+      p->steps[full ? TINY_FWD_FULL : TINY_FWD].push_back(s);
+    }
+    // one step alone gains nothing
+    if (order.size() < 2) {
+      p->steps[full ? TINY_FWD_FULL : TINY_FWD].clear();
+      for (int j : order) (full ? p->nodes[j].tiny_full : p->nodes[j].tiny) = false;
+    }
+  }
+  // reverse: below[j] = every gradient step of j's subtree (j's own included) is tiny
+  const bool cplx = p->dt == OME_C32 || p->dt == OME_C64;
+  std::vector<char> below(nn, 0);
+  p->rev_tiny.resize(nn);
+  for (int j = 0; j < nn; ++j) {
+    const PNode& n = p->nodes[j];
+    bool all = true;
+    p->rev_tiny[j].assign(n.args.size(), 0);
+    for (size_t i = 0; i < n.args.size(); ++i) {
+      std::vector<std::vector<int32_t>> xs;
+      for (size_t a = 0; a < n.args.size(); ++a) xs.push_back(a == i ? n.iy : labels(n.args[a], false));
+      const int r = n.args[i];
+      const bool t = tiny_step(p, xs, labels(r, false)) && (r < 0 || below[r]);
+      p->rev_tiny[j][i] = t;
+      all = all && t;
+    }
+    below[j] = all;
+  }
+  std::vector<int> lev(nn, 0);   // reverse level of a node's own steps
+  for (int j = root; j >= 0; --j) {
+    const PNode& n = p->nodes[j];
+    for (size_t i = 0; i < n.args.size(); ++i) {
+      if (!p->rev_tiny[j][i]) continue;
+      TinyStep s;
+      s.nin = (int)n.args.size();
+      s.level = lev[j];
+      for (int a = 0; a < s.nin; ++a) {
+        const int r = n.args[a];
+        s.kind[a] = a == (int)i ? TinyStep::GRAD : r >= 0 ? TinyStep::VALUE : TinyStep::INPUT;
+        s.ref[a] = a == (int)i ? j : r >= 0 ? r : -r - 1;
+      }
+      const int r = n.args[i];
+      s.kind[2] = r >= 0 ? TinyStep::GRAD : TinyStep::INPUT_GRAD;
+      s.ref[2] = r >= 0 ? r : -r - 1;
+      if (cplx) s.flags = TINY_CONJY | (i == 0 ? TINY_CONJ0 : TINY_CONJ1);
+      if (r >= 0) lev[r] = lev[j] + 1;
+      p->steps[TINY_REV].push_back(s);
+    }
+  }
+  std::stable_sort(p->steps[TINY_REV].begin(), p->steps[TINY_REV].end(),
+                   [](const TinyStep& a, const TinyStep& b) { return a.level < b.level; });
+}
+
 }  // namespace
 
 extern "C" {
@@ -270,16 +423,25 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
       delete p;
       return set_err(OME_INVALID_ARGUMENT, "node %d is not reachable from the root", j);
     }
+  plan_tiny(p);
   // forward arena (sliced shapes), liveness: a node's output dies when its
-  // parent ran.  The FP64 cross-slice accumulator lives through every slice,
+  // parent ran.  The tiny nodes run before all others, in any order among
+  // themselves, so their buffers are reserved together.  The FP64 cross-slice accumulator lives through every slice,
   // so it is reserved first and never shared with a node buffer.
   const int root = nnodes - 1;
   const bool sliced = !p->sliced.empty();
   p->acc64 = sliced && (dtype == OME_F32 || dtype == OME_F64 || dtype == OME_C32);
   Arena ar;
   if (p->acc64) p->acc_off = ar.alloc((size_t)p->nodes[root].numel * (dtype == OME_C32 ? 16 : 8));
+  for (int j = 0; j < root; ++j)
+    if (p->nodes[j].tiny) p->nodes[j].off_fwd = ar.alloc((size_t)p->nodes[j].numel_s * p->esize);
+  for (int j = 0; j < root; ++j)
+    if (p->nodes[j].tiny)
+      for (int r : p->nodes[j].args)
+        if (r >= 0) ar.release(p->nodes[r].off_fwd);
   for (int j = 0; j < root; ++j) {
     PNode& n = p->nodes[j];
+    if (n.tiny) continue;
     n.off_fwd = ar.alloc((size_t)n.numel_s * p->esize);
     for (int r : n.args)
       if (r >= 0) ar.release(p->nodes[r].off_fwd);
@@ -441,6 +603,127 @@ int run_node(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int j, const Leaves& inp
 size_t off_fwd_of(const PNode& n) { return n.off_fwd; }
 size_t off_keep_of(const PNode& n) { return n.off_keep; }
 
+// The descriptors of a tiny program for the caller's input strides, from the
+// plan's cache or built now (pointers are set per launch).
+std::shared_ptr<const TinyProgram> tiny_program(ome_plan* p, int which, const Leaves& in) {
+  size_t ns = 0;
+  for (auto& l : p->in_labels) ns += l.size();
+  {
+    std::lock_guard<std::mutex> lk(p->prog_mutex);
+    const auto& c = p->prog[which];
+    if (c && c->strided == (in.str != nullptr) &&
+        (!in.str || std::equal(c->strides.begin(), c->strides.end(), in.str)))
+      return c;
+  }
+  auto prog = std::make_shared<TinyProgram>();
+  prog->strided = in.str != nullptr;
+  if (in.str) prog->strides.assign(in.str, in.str + ns);
+  prog->ok = true;
+  const bool sliced = which == TINY_FWD;
+  static const std::vector<int32_t> none;
+  const std::vector<int64_t> fix(p->sliced.size(), 0);
+  const std::vector<int32_t>& drop = sliced ? p->sliced : none;
+  std::vector<const void*> null((size_t)p->ninputs, nullptr);
+  const Leaves nowhere{null.data(), in.str};
+  for (const TinyStep& st : p->steps[which]) {
+    HView xs[2], y;
+    for (int a = 0; a < st.nin; ++a)
+      xs[a] = st.kind[a] == TinyStep::INPUT
+                  ? leaf_view(p, nowhere, st.ref[a], drop, fix)
+                  : make_view(p, nullptr, sliced ? p->nodes[st.ref[a]].iy_s : p->nodes[st.ref[a]].iy, none, fix);
+    y = st.kind[2] == TinyStep::INPUT_GRAD
+            ? make_view(p, nullptr, p->in_labels[st.ref[2]], none, fix)
+            : make_view(p, nullptr, sliced ? p->nodes[st.ref[2]].iy_s : p->nodes[st.ref[2]].iy, none, fix);
+    TinyNode n;
+    if (!tiny_node(n, st.nin, xs, y)) {
+      prog->ok = false;
+      break;
+    }
+    n.flags |= st.flags;
+    prog->nodes.push_back(n);
+    prog->level.push_back(st.level);
+  }
+  std::lock_guard<std::mutex> lk(p->prog_mutex);
+  p->prog[which] = prog;
+  return prog;
+}
+
+// Runs a tiny program; *done = false (nothing launched) if the input strides
+// do not fit its descriptors.  y: where a tree that is tiny as a whole puts
+// its value (NULL: the root is left out).
+int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves& in, const std::vector<int64_t>& fix,
+             char* y, char* dy_root, void* const* dxs, bool* done) {
+  *done = true;
+  const auto& steps = p->steps[which];
+  if (steps.empty()) return OME_OK;
+  auto prog = tiny_program(p, which, in);
+  *done = prog->ok;
+  if (!prog->ok) return OME_OK;
+  const bool keep = which != TINY_FWD;
+  const int root = (int)p->nodes.size() - 1;
+  // element offsets of the inputs at this slice
+  std::vector<int64_t> off((size_t)p->ninputs, 0);
+  if (which == TINY_FWD && !p->sliced.empty())
+    for (int t = 0; t < p->ninputs; ++t) {
+      int64_t st = 1;
+      for (size_t d = 0; d < p->in_labels[t].size(); ++d) {
+        const int32_t l = p->in_labels[t][d];
+        auto it = std::find(p->sliced.begin(), p->sliced.end(), l);
+        if (it != p->sliced.end())
+          off[t] += fix[it - p->sliced.begin()] * (in.str ? in.str[p->in_pos[t] + (int)d] : st);
+        st *= p->ext.at(l);
+      }
+    }
+  auto at = [&](TinyStep::Kind k, int ref) -> char* {
+    switch (k) {
+      case TinyStep::VALUE: return ctx->ws + (keep ? p->nodes[ref].off_keep : p->nodes[ref].off_fwd);
+      case TinyStep::GRAD: return ref == root ? dy_root : ctx->ws + p->nodes[ref].off_grad;
+      case TinyStep::INPUT: return (char*)in.data[ref] + off[ref] * (int64_t)p->esize;
+      case TinyStep::OUTPUT: return y;
+      default: return (char*)dxs[ref];
+    }
+  };
+  std::vector<TinyNode> nodes(prog->nodes);
+  size_t count = steps.size();
+  if (steps.back().kind[2] == TinyStep::OUTPUT && !y) --count;
+  for (size_t i = 0; i < count; ++i) {
+    const TinyStep& st = steps[i];
+    nodes[i].x0 = at(st.kind[0], st.ref[0]);
+    nodes[i].x1 = st.nin > 1 ? at(st.kind[1], st.ref[1]) : nullptr;
+    nodes[i].y = at(st.kind[2], st.ref[2]);
+  }
+  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)count, s), "tiny program");
+}
+
+// The forward values of every node but the root: the tiny program, then the
+// other nodes in post-order.  y: the tree's output if its value goes there as
+// it is; *rooted = true if the program has put it there.
+int run_forward(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves& inputs,
+                const std::vector<int64_t>& fix, size_t scratch, char* y, bool* rooted) {
+  const bool sliced = which == TINY_FWD && !p->sliced.empty(), keep = which != TINY_FWD;
+  static const std::vector<int32_t> none;
+  static const std::vector<int64_t> nofix;
+  const Scalar one = scalar_one(p->dt), zero = scalar_zero(p->dt);
+  const int root = (int)p->nodes.size() - 1;
+  bool done = false;
+  int rc = run_tiny(ctx, p, s, which, inputs, fix, y, nullptr, nullptr, &done);
+  if (rc) return rc;
+  *rooted = done && y && !p->steps[which].empty() && p->steps[which].back().kind[2] == TinyStep::OUTPUT;
+  auto one_node = [&](int j) {
+    const PNode& n = p->nodes[j];
+    HView v = make_view(p, ctx->ws + (keep ? n.off_keep : n.off_fwd), sliced ? n.iy_s : n.iy, none, nofix);
+    return run_node(ctx, p, s, j, inputs, sliced, fix, keep ? off_keep_of : off_fwd_of, v, one, zero, scratch);
+  };
+  for (int pass = done ? 1 : 0; pass < 2; ++pass)
+    for (int j = 0; j < root; ++j) {
+      const bool tiny = keep ? p->nodes[j].tiny_full : p->nodes[j].tiny;
+      if (tiny != (pass == 0)) continue;
+      rc = one_node(j);
+      if (rc) return rc;
+    }
+  return OME_OK;
+}
+
 
 // Slices [b, e) of the tree, each root result added at its sliced output
 // positions: into the F64/C64 buffer `acc` for acc64 plans (the root goes to
@@ -463,14 +746,12 @@ int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, 
       fix[i] = r % ext;
       r /= ext;
     }
-    for (int j = 0; j < root; ++j) {
-      HView v = make_view(p, ctx->ws + p->nodes[j].off_fwd, p->nodes[j].iy_s, none, nofix);
-      int rc = run_node(ctx, p, s, j, inputs, true, fix, off_fwd_of, v, one, zero, scratch);
-      if (rc) return rc;
-    }
+    bool rooted;
+    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, fix, scratch, nullptr, &rooted);
+    if (rc) return rc;
     if (p->acc64) {
       HView tv = make_view(p, ctx->ws + p->tmp_off, rn.iy_s, none, nofix);
-      int rc = run_node(ctx, p, s, root, inputs, true, fix, off_fwd_of, tv, one, zero, scratch);
+      rc = run_node(ctx, p, s, root, inputs, true, fix, off_fwd_of, tv, one, zero, scratch);
       if (rc) return rc;
       // acc[slice positions] += temp
       const size_t w = dt == OME_C32 ? 16 : 8;
@@ -482,7 +763,7 @@ int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, 
       if (rc) return rc;
     } else {
       HView yv = make_view(p, acc, rn.iy, p->sliced, fix);
-      int rc = run_node(ctx, p, s, root, inputs, true, fix, off_fwd_of, yv, sx, one, scratch);
+      rc = run_node(ctx, p, s, root, inputs, true, fix, off_fwd_of, yv, sx, one, scratch);
       if (rc) return rc;
     }
   }
@@ -515,11 +796,10 @@ int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void
   static const std::vector<int64_t> nofix;
 
   if (p->sliced.empty()) {
-    for (int j = 0; j < root; ++j) {
-      HView v = make_view(p, ctx->ws + p->nodes[j].off_fwd, p->nodes[j].iy, none, nofix);
-      int rc = run_node(ctx, p, s, j, inputs, false, nofix, off_fwd_of, v, one, zero, scratch);
-      if (rc) return rc;
-    }
+    bool rooted;
+    const bool plain = scalar_is_one(dt, sx) && scalar_is_zero(dt, sy);
+    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, nofix, scratch, plain ? (char*)y : nullptr, &rooted);
+    if (rc || rooted) return rc;
     HView yv = make_view(p, (char*)y, rn.iy, none, nofix);
     return run_node(ctx, p, s, root, inputs, false, nofix, off_fwd_of, yv, sx, sy, scratch);
   }
@@ -641,13 +921,11 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
   static const std::vector<int64_t> nofix;
   const size_t scratch = (p->grad_arena + 255) & ~(size_t)255;
   // forward, every value kept
-  for (int j = 0; j < root; ++j) {
-    HView v = make_view(p, ctx->ws + p->nodes[j].off_keep, p->nodes[j].iy, none, nofix);
-    int rc = run_node(ctx, p, s, j, inputs, false, nofix, off_keep_of, v, one, zero, scratch);
-    if (rc) return rc;
-  }
+  bool rooted;
+  int rc = run_forward(ctx, p, s, TINY_FWD_FULL, inputs, nofix, scratch, (char*)y, &rooted);
+  if (rc) return rc;
   HView yv = make_view(p, (char*)y, rn.iy, none, nofix);
-  int rc = run_node(ctx, p, s, root, inputs, false, nofix, off_keep_of, yv, one, zero, scratch);
+  if (!rooted) rc = run_node(ctx, p, s, root, inputs, false, nofix, off_keep_of, yv, one, zero, scratch);
   if (rc) return rc;
   // root cotangent: ones (init_gradient, src/bp.jl:133-138) or the caller's dy
   char* dy_root;
@@ -662,13 +940,16 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
     if (rc) return rc;
   }
   const size_t scratch2 = ctx->ws_top;
-  // reverse sweep
+  // reverse sweep: the steps above, then the tiny program of the steps below
+  // (all in node order if its descriptors do not fit the input strides)
+  bool tiny = !p->steps[TINY_REV].empty() && tiny_program(p, TINY_REV, inputs)->ok;
   for (int j = root; j >= 0; --j) {
     const PNode& n = p->nodes[j];
     char* gj = j == root ? dy_root : ctx->ws + n.off_grad;
     // conj(dy) in place (complex): gradients are conj(einsum(.., conj(dy), ..))
     const int nin = (int)n.args.size();
     for (int i = 0; i < nin; ++i) {
+      if (tiny && p->rev_tiny[j][i]) continue;
       HView xs[MAXIN];
       for (int a = 0; a < nin; ++a) {
         const int r = n.args[a];
@@ -704,6 +985,7 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
       }
     }
   }
+  if (tiny) return run_tiny(ctx, p, s, TINY_REV, inputs, nofix, nullptr, dy_root, dxs, &tiny);
   return OME_OK;
 }
 
