@@ -560,23 +560,31 @@ cudaError_t launch_gemm_split(const GemmArgs& g, int nterms, void* workspace, si
 //
 // k_pack_split writes each operand once as BF16 terms, already in the UMMA
 // K-major canonical layout: for every (batch, 128-row tile, 32-wide k-step)
-// one contiguous blob of NT 8 KB term tiles.  The GEMM then moves a whole
-// stage with two cp.async.bulk copies (no tensor map, no converter warps):
-//  * warp 8 lane 0 (producer) issues the bulk copies into a STAGES-deep ring,
-//    completion counted by the stage's mbarrier (expect_tx);
-//  * warp 9 allocates TMEM; its lane 0 issues the MMAs exactly as
-//    k_gemm_bf16x3 does (main t0*t0 and cross-term accumulators, two TMEM
-//    buffers, a fresh accumulation every CHUNK k-steps);
-//  * warps 0-7 drain each finished chunk (tcgen05.ld) into FP32 running sums
-//    held in registers (thread = one row x 64 columns), round-to-nearest
-//    adds, and store the tile (αβ epilogue, or a split partial).
+// one contiguous blob of NT 8 KB term tiles.  The GEMM (a cluster of two CTAs
+// per 256 x 256 tile, tcgen05.mma.cta_group::2, M = N = 256) then moves a stage
+// with one bulk copy per operand (no tensor map, no converter warps):
+//  * warp 8 lane 0 of each CTA (producer) issues its CTA's copies into a
+//    STAGES-deep ring: the 128 rows of A that its TMEM accumulates and its half
+//    of B's 256 columns; completion is counted by the stage's mbarrier;
+//  * warp 9 allocates TMEM; in the leader CTA it issues the MMAs (one elected
+//    lane), in the peer it tells the leader that a stage has landed;
+//  * TMEM holds one main (t0*t0) and one cross-term accumulator of 256 columns.
+//    A stage's cross products go first: while they run, warps 0-7 of both CTAs
+//    drain the main accumulator of the chunk before (CHUNK stages) into FP32
+//    running sums in registers (thread = one row x 128 columns) with
+//    round-to-nearest adds.  The cross terms are 2^-8 of the main ones and so is
+//    the round-off of their accumulation: they are drained every fourth chunk;
+//  * the same warps store the tile (αβ epilogue, or a split partial).
 // The kernel is persistent over work units: the first F tiles (whole waves of
-// the grid) are computed whole, the remaining tiles are cut into S K-splits so
-// that the last wave fills the SMs; split partials are summed in split order
-// by k_splitk_tiles (deterministic).  The chunk counter runs across units, so
+// the clusters) are computed whole, the remaining tiles are cut into S K-splits
+// so that the last wave fills the SMs; split partials are summed in split order
+// by k_splitk_tiles (deterministic).  The chunk counters run across units, so
 // the epilogue of one unit overlaps the MMAs of the next.
+// Bound by the tensor pipe.  An MMA of the pair takes 155 clocks with N = 128 and
+// 185 with N = 256 (copies, drains, operand layout and the accumulators' order
+// changed neither), so the tile is the widest there is.
 namespace pk {
-constexpr int BM = 128, BN = 128, BK = 32, CHUNK = 8;
+constexpr int BM = 128, BK = 32, CHUNK = 4, XCHUNK = 4 * CHUNK;
 constexpr int TILE_BYTES = BM * BK * 2;     // one term of one operand for one k-step
 constexpr int NDRAIN = 256;                 // drain / epilogue warps 0-7
 constexpr int NTHREADS = NDRAIN + 64;       // + producer warp 8 + MMA warp 9
@@ -585,8 +593,12 @@ template <int NT> struct Cfg {
   static constexpr int BLOB = NT * TILE_BYTES;
   static constexpr int STAGE_BYTES = 2 * BLOB;
   static constexpr int STAGES = NT == 2 ? 6 : 4;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256;
+  static constexpr int OUT_BYTES = NDRAIN * 32 * 4;       // 32 columns of every drain thread on their way to C
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + OUT_BYTES;
 };
+// kind::f16, BF16 x BF16 -> F32, K-major A and B, M = 256 (CTA pair), N = 256
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
+                           ((uint32_t)(256 >> 4) << 24);
 }  // namespace pk
 
 struct PackArgs {
@@ -603,7 +615,8 @@ struct PkArgs {
   GemmArgs g;                  // C, M, N, L and the epilogue
   const unsigned char* PA;     // packed A [L][TM][NKT]
   const unsigned char* PB;     // packed B [L][TN][NKT]
-  float* partial;              // [(tiles - F) * S][BN][BM]
+  float* partial;              // [(tiles - F) * S][256 n][256 m]
+  int64_t RA, RB;              // 128-row tiles of A and B
   int64_t TM, TN, NKT, tiles, F, ksplit, units;
   int S;
 };
@@ -685,415 +698,6 @@ __device__ __forceinline__ void mbar_wait_quiesce(uint64_t* bar, uint32_t parity
     }
 }
 
-template <int NT>
-__global__ void __launch_bounds__(pk::NTHREADS, 1) k_gemm_packed(const __grid_constant__ PkArgs t) {
-  using namespace pk;
-  constexpr int STAGES = Cfg<NT>::STAGES, STAGE_BYTES = Cfg<NT>::STAGE_BYTES, BLOB = Cfg<NT>::BLOB;
-  extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* chunk_done = empty + STAGES;   // [2]
-  uint64_t* drained = chunk_done + 2;      // [2]
-  uint64_t* final_bar = drained + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const GemmArgs& g = t.g;
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&chunk_done[b], 1);
-      mbar_init(&drained[b], NDRAIN);
-    }
-    mbar_init(final_bar, 1);
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 9) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  auto tmem_main = [&](int b) { return tmem + (uint32_t)(256 * b); };
-  auto tmem_cross = [&](int b) { return tmem + (uint32_t)(256 * b + 128); };
-  const uint32_t sbase = smem_u32(smem);
-
-  // unit u -> tile (l, mt, nt; mt fastest), k-step range, split slot (-1: whole)
-  auto decode = [&](int64_t u, int64_t& l, int64_t& mt, int64_t& nt, int64_t& kb, int64_t& ke, int64_t& slot) {
-    int64_t tile;
-    if (u < t.F) {
-      tile = u; kb = 0; ke = t.NKT; slot = -1;
-    } else {
-      const int64_t v = u - t.F;
-      tile = t.F + v / t.S;
-      kb = (v % t.S) * t.ksplit;
-      ke = min(t.NKT, kb + t.ksplit);
-      slot = v;
-    }
-    mt = tile % t.TM;
-    const int64_t r = tile / t.TM;
-    nt = r % t.TN;
-    l = r / t.TN;
-  };
-
-  if (warp == 8) {
-    // ---------------- producer: two bulk copies per stage ----------------
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int64_t u = blockIdx.x; u < t.units; u += gridDim.x) {
-        int64_t l, mt, nt, kb, ke, slot;
-        decode(u, l, mt, nt, kb, ke, slot);
-        const unsigned char* pa = t.PA + ((l * t.TM + mt) * t.NKT) * (int64_t)BLOB;
-        const unsigned char* pb = t.PB + ((l * t.TN + nt) * t.NKT) * (int64_t)BLOB;
-        bool ok = true;
-        for (int64_t kt = kb; kt < ke; ++kt, ++it) {
-          const int s = it % STAGES;
-          if (it >= (uint32_t)STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag)) {
-            ok = false;
-            break;
-          }
-          mbar_expect_tx(&full[s], 2 * BLOB);
-          bulk_g2s(sbase + s * STAGE_BYTES, pa + kt * BLOB, BLOB, &full[s]);
-          bulk_g2s(sbase + s * STAGE_BYTES + BLOB, pb + kt * BLOB, BLOB, &full[s]);
-        }
-        if (!ok) break;
-      }
-      // the copies of the last STAGES issues must land before the block exits
-      for (uint32_t i = it > (uint32_t)STAGES ? it - STAGES : 0; i < it; ++i)
-        mbar_wait_quiesce(&full[i % STAGES], (i / STAGES) & 1);
-    }
-  } else if (warp == 9) {
-    // ---------------- MMA issue ----------------
-    if (lane == 0) {
-      uint32_t it = 0, gc = 0;
-      bool ok = true;
-      for (int64_t u = blockIdx.x; u < t.units && ok; u += gridDim.x) {
-        int64_t l, mt, nt, kb, ke, slot;
-        decode(u, l, mt, nt, kb, ke, slot);
-        const int nk = (int)(ke - kb);
-        for (int j = 0; j < nk; ++j, ++it) {
-          const uint32_t c = gc + j / CHUNK;
-          const int b = c & 1;
-          const bool first = j % CHUNK == 0;
-          if (first && c >= 2 && !mbar_wait(&drained[b], ((c >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-          const int s = it % STAGES;
-          if (!mbar_wait(&full[s], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sb = sbase + s * STAGE_BYTES;
-#pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {
-            const uint32_t off = kk * 256;
-            uint64_t ad[NT], bd[NT];
-#pragma unroll
-            for (int q = 0; q < NT; ++q) {
-              ad[q] = umma_desc(sb + q * TILE_BYTES + off);
-              bd[q] = umma_desc(sb + BLOB + q * TILE_BYTES + off);
-            }
-            const uint32_t keep = (first && kk == 0) ? 0u : 1u;
-            umma_bf16(tmem_main(b), ad[0], bd[0], keep);
-            bool first_cross = true;
-#pragma unroll
-            for (int d = 1; d < NT; ++d)
-#pragma unroll
-              for (int i = 0; i <= d; ++i) {
-                umma_bf16(tmem_cross(b), ad[i], bd[d - i], first_cross ? keep : 1u);
-                first_cross = false;
-              }
-          }
-          umma_commit(&empty[s]);
-          if (j % CHUNK == CHUNK - 1 || j == nk - 1) umma_commit(&chunk_done[b]);
-        }
-        gc += (uint32_t)((nk + CHUNK - 1) / CHUNK);
-      }
-      // every MMA this thread issued must finish before TMEM is freed
-      umma_commit(final_bar);
-      mbar_wait_quiesce(final_bar, 0);
-    }
-  } else {
-    // ---------------- drain + epilogue (warps 0-7) ----------------
-    const int q = warp & 3, h = warp >> 2;
-    const int row = 32 * q + lane;
-    const int col0 = 64 * h;
-    const uint32_t lane_off = (uint32_t)(32 * q) << 16;
-    uint32_t gc = 0;
-    const float sx = scalar_as<float>(g.sx), sy = scalar_as<float>(g.sy);
-    float* Cp = static_cast<float*>(g.C);
-    for (int64_t u = blockIdx.x; u < t.units; u += gridDim.x) {
-      int64_t l, mt, nt, kb, ke, slot;
-      decode(u, l, mt, nt, kb, ke, slot);
-      const int nch = (int)((ke - kb + CHUNK - 1) / CHUNK);
-      float sum[64];
-#pragma unroll
-      for (int j = 0; j < 64; ++j) sum[j] = 0.f;
-      bool ok = true;
-      for (int ci = 0; ci < nch; ++ci, ++gc) {
-        const int b = gc & 1;
-        if (!mbar_wait(&chunk_done[b], (gc >> 1) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-          uint32_t rm[16], rc[16];
-          __syncwarp();
-          tmem_ld16(tmem_main(b) + lane_off + (uint32_t)(col0 + 16 * hh), rm);
-          tmem_ld16(tmem_cross(b) + lane_off + (uint32_t)(col0 + 16 * hh), rc);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float v = __uint_as_float(rm[j]) + __uint_as_float(rc[j]);
-            sum[16 * hh + j] = ci == 0 ? v : sum[16 * hh + j] + v;
-          }
-        }
-        tc_fence_before();
-        mbar_arrive(&drained[b]);
-      }
-      if (!ok) break;
-      if (slot >= 0) {
-        float* pp = t.partial + (slot * BN + col0) * (int64_t)BM + row;
-#pragma unroll
-        for (int j = 0; j < 64; ++j) pp[(int64_t)j * BM] = sum[j];
-      } else {
-        const int64_t m = mt * BM + row;
-        if (m < g.M) {
-          const int64_t base = mode_offset(l, g.nl, g.l_ext, g.l_sc) + c_moff(g, m);
-          const int64_t n0 = nt * BN + col0;
-#pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            const int64_t n = n0 + j;
-            if (n < g.N) {
-              float* cp = Cp + base + c_noff(g, n);
-              float o = g.sx_one ? sum[j] : sx * sum[j];
-              if (!g.sy_zero) o = fmaf(sy, *cp, o);
-              *cp = o;
-            }
-          }
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 9) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(pk::TMEM_COLS) : "memory");
-  }
-}
-
-// Sum the S split partials of each split tile in split order; αβ epilogue.
-__global__ void __launch_bounds__(256) k_splitk_tiles(const __grid_constant__ PkArgs t) {
-  using namespace pk;
-  const GemmArgs& g = t.g;
-  const float sx = scalar_as<float>(g.sx), sy = scalar_as<float>(g.sy);
-  float* Cp = static_cast<float*>(g.C);
-  const int64_t total = (t.tiles - t.F) * BM * BN;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t mloc = i % BM;
-    const int64_t r = i / BM;
-    const int64_t nloc = r % BN;
-    const int64_t v = r / BN;
-    const int64_t tile = t.F + v;
-    const int64_t mt = tile % t.TM, r2 = tile / t.TM, nt = r2 % t.TN, l = r2 / t.TN;
-    const int64_t m = mt * BM + mloc, n = nt * BN + nloc;
-    if (m >= g.M || n >= g.N) continue;
-    float acc = 0.f;
-    for (int s = 0; s < t.S; ++s) acc += t.partial[((v * t.S + s) * BN + nloc) * BM + mloc];
-    float* cp = Cp + mode_offset(l, g.nl, g.l_ext, g.l_sc) + c_moff(g, m) +
-                c_noff(g, n);
-    float o = g.sx_one ? acc : sx * acc;
-    if (!g.sy_zero) o = fmaf(sy, *cp, o);
-    *cp = o;
-  }
-}
-
-static void pack_args(PackArgs& p, const float* X, unsigned char* P, int64_t R, int nr, const int64_t* r_ext,
-                      const int64_t* r_str, const GemmArgs& g, const int64_t* k_str, const int64_t* l_str) {
-  memset(&p, 0, sizeof(p));
-  p.X = X;
-  p.P = P;
-  p.R = R;
-  p.K = g.K;
-  p.L = g.L;
-  p.RT = (R + pk::BM - 1) / pk::BM;
-  p.NKT = (g.K + pk::BK - 1) / pk::BK;
-  p.nr = nr;
-  p.nk = g.nk;
-  p.nl = g.nl;
-  for (int i = 0; i < nr; ++i) { p.r_ext[i] = r_ext[i]; p.r_str[i] = r_str[i]; }
-  for (int i = 0; i < g.nk; ++i) { p.k_ext[i] = g.k_ext[i]; p.k_str[i] = k_str[i]; }
-  for (int i = 0; i < g.nl; ++i) { p.l_ext[i] = g.l_ext[i]; p.l_str[i] = l_str[i]; }
-  p.kfast = k_str[0] == 1 && g.k_ext[0] % 8 == 0;
-}
-
-size_t gemm_packed_bytes(const GemmArgs& g, int nterms, int num_sms) {
-  using namespace pk;
-  const int64_t TM = (g.M + BM - 1) / BM, TN = (g.N + BN - 1) / BN, NKT = (g.K + BK - 1) / BK;
-  const size_t blob = (size_t)nterms * TILE_BYTES;
-  // packed operands + at most one grid's worth of split partials
-  return (size_t)g.L * (TM + TN) * NKT * blob + (size_t)num_sms * BM * BN * 4 + 1024;
-}
-
-cudaError_t launch_gemm_packed(const GemmArgs& g, int nterms, void* workspace, size_t ws_bytes, int num_sms,
-                               cudaStream_t s, int64_t* ctab) {
-  using namespace pk;
-  if (!gemm_split_supported(g) || (nterms != 2 && nterms != 3)) return cudaErrorNotSupported;
-  static std::atomic<unsigned long long> attr2{0}, attr3{0};
-  {
-    const cudaError_t e = nterms == 2 ? set_smem_once(attr2, k_gemm_packed<2>, Cfg<2>::SMEM_BYTES)
-                                      : set_smem_once(attr3, k_gemm_packed<3>, Cfg<3>::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-  }
-  const int64_t TM = (g.M + BM - 1) / BM, TN = (g.N + BN - 1) / BN, NKT = (g.K + BK - 1) / BK;
-  const size_t blob = (size_t)nterms * TILE_BYTES;
-  const size_t bytes_a = (size_t)g.L * TM * NKT * blob, bytes_b = (size_t)g.L * TN * NKT * blob;
-  const int64_t tiles = g.L * TM * TN;
-  const int64_t G = num_sms;
-  // whole tiles for every complete wave; the rest split along K so that the
-  // last wave covers the grid (at least 8 k-steps per split)
-  int64_t F = tiles >= G ? (tiles / G) * G : 0;
-  int64_t Rt = tiles - F;
-  int64_t S = 1;
-  if (Rt > 0) {
-    S = std::max<int64_t>(1, G / Rt);
-    S = std::min<int64_t>(S, std::max<int64_t>(1, NKT / 8));
-  }
-  const int64_t ksplit = (NKT + S - 1) / S;
-  S = (NKT + ksplit - 1) / ksplit;
-  if (S == 1) {
-    F = tiles;
-    Rt = 0;
-  }
-  const size_t bytes_p = (size_t)Rt * S * BM * BN * 4;
-  if (bytes_a + bytes_b + bytes_p + 768 > ws_bytes) return cudaErrorNotSupported;
-  unsigned char* w = static_cast<unsigned char*>(workspace);
-  unsigned char* PA = w;
-  unsigned char* PB = w + ((bytes_a + 255) & ~(size_t)255);
-  float* part = reinterpret_cast<float*>(PB + ((bytes_b + 255) & ~(size_t)255));
-
-  PackArgs pa, pb;
-  pack_args(pa, static_cast<const float*>(g.A), PA, g.M, g.nm, g.m_ext, g.m_sa, g, g.k_sa, g.l_sa);
-  pack_args(pb, static_cast<const float*>(g.B), PB, g.N, g.nn, g.n_ext, g.n_sb, g, g.k_sb, g.l_sb);
-  if (ctab) {
-    pa.c_tab = ctab;
-    pb.c_tab = ctab + g.M;
-    for (int i = 0; i < g.nm; ++i) pa.c_str[i] = g.m_sc[i];
-    for (int i = 0; i < g.nn; ++i) pb.c_str[i] = g.n_sc[i];
-  }
-  const int64_t units = g.L * (TM + TN) * NKT + (ctab ? (g.M + 255) / 256 + (g.N + 255) / 256 : 0);
-  const unsigned gp = (unsigned)std::min<int64_t>(units, (int64_t)num_sms * 8);
-  if (nterms == 2) k_pack_split<2><<<gp, 256, 0, s>>>(pa, pb);
-  else k_pack_split<3><<<gp, 256, 0, s>>>(pa, pb);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-
-  PkArgs t;
-  memset(&t, 0, sizeof(t));
-  t.g = g;
-  if (ctab) {
-    t.g.m_tab_c = ctab;
-    t.g.n_tab_c = ctab + g.M;
-  }
-  t.PA = PA;
-  t.PB = PB;
-  t.partial = part;
-  t.TM = TM;
-  t.TN = TN;
-  t.NKT = NKT;
-  t.tiles = tiles;
-  t.F = F;
-  t.S = (int)S;
-  t.ksplit = ksplit;
-  t.units = F + Rt * S;
-  const unsigned grid = (unsigned)std::min<int64_t>(t.units, G);
-  // plain launches: a GEMM block started early would hold its SM's shared
-  // memory and TMEM while waiting, which stalls other streams' kernels
-  {
-    KernelTimer kt(s, "k_gemm_packed");
-    if (nterms == 2) k_gemm_packed<2><<<grid, NTHREADS, Cfg<2>::SMEM_BYTES, s>>>(t);
-    else k_gemm_packed<3><<<grid, NTHREADS, Cfg<3>::SMEM_BYTES, s>>>(t);
-  }
-  count_launch();
-  e = cudaGetLastError();
-  if (e != cudaSuccess || Rt == 0) return e;
-  const int64_t total = Rt * BM * BN;
-  const int64_t nb = (total + 255) / 256;
-  k_splitk_tiles<<<(unsigned)std::min<int64_t>(nb, (int64_t)num_sms * 16), 256, 0, s>>>(t);
-  count_launch();
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// k_gemm_tma2: 2-SM tensor-core GEMM fed by tensor maps over the FP32 inputs.
-//
-// The operands are read in place, through TMA tensor maps whose dimensions
-// and strides are the contraction's merged mode groups (the permutation of
-// simplifyto, src/einsum.jl:127-134, lives in the maps: nothing is written
-// back to HBM), and split into BF16 terms in shared memory.
-//  * A cluster of two CTAs computes a 256 x 256 tile of C with
-//    tcgen05.mma.cta_group::2 (M = 256, N = 256, K = 16): CTA r holds rows
-//    128r..128r+127 of the A tile and columns 128r..128r+127 of the B tile;
-//    its TMEM receives rows 128r.. of the accumulator, all 256 columns.
-//  * Warp 16 (one thread) issues, per 32-wide k stage, the TMA loads of this
-//    CTA's FP32 A and B tiles (128-byte swizzle, zero fill past the extents;
-//    no multicast) into one of three FP32 stages.
-//  * Warps 0-7 (A) and 8-15 (B) convert a stage into NT BF16 terms per value
-//    in the UMMA K-major canonical layout (conflict-free shared-memory reads
-//    and writes in both operand orientations), then arrive on the leader
-//    CTA's term_full barrier (remote arrive, release at cluster scope).
-//  * Warp 17 of the leader CTA issues the MMAs (main t0*t0 and cross-term
-//    accumulators, 2 x 256 TMEM columns) and releases each term stage to both
-//    CTAs with a multicast tcgen05.commit.
-//  * Every CHS stages the 16 converter warps of both CTAs drain the
-//    accumulators (tcgen05.ld) into FP32 running sums in registers with
-//    round-to-nearest adds; the accumulators are single-buffered, so the
-//    converters drain chunk c before they wait for a term stage whose MMAs
-//    come after it (no cycle in the waits).
-//  * Persistent over units: whole 256 x 256 tiles for the complete waves of
-//    clusters, the last wave's tiles cut along K (partials summed in split
-//    order by k_splitk_tiles2: deterministic).
-//  * Every wait is bounded (tc::WAIT_NS); on expiry the CTA records the
-//    timeout flag, stops waiting, lets its own copies and MMAs finish and
-//    frees its TMEM.  Both CTAs meet at a final cluster barrier.
-namespace t2 {
-constexpr int BM = 128;                    // rows per CTA (256 per cluster tile)
-constexpr int BK = 32;                     // k per stage
-constexpr int CHS = 8;                     // stages per accumulator chunk (16 k-steps)
-constexpr int F32_STAGES = 2;
-constexpr int NSR = 32;                    // running sums per thread in registers (the other 32 in shared memory)
-constexpr int F32_TILE = BM * BK * 4;      // 16 KB: one operand, one stage
-constexpr int TERM_TILE = BM * BK * 2;     // 8 KB: one term of one operand
-constexpr int NCONV = 512;                 // converter + drain warps 0-15
-constexpr int NTHREADS = NCONV + 64;       // + TMA warp 16 + MMA warp 17
-constexpr int TMEM_COLS = 512;
-template <int NT> struct Cfg {
-  static constexpr int F32_STAGE = 2 * F32_TILE;          // A tile, B tile
-  static constexpr int TERM_STAGE = 2 * NT * TERM_TILE;   // A terms, B terms
-  static constexpr int TSTAGES = NT == 2 ? 3 : 2;
-  static constexpr int SUM_BYTES = NCONV * (64 - NSR) * 4;   // 64 KB of running sums
-  static constexpr int BAR_BYTES = 256;
-  static constexpr int SMEM_BYTES = F32_STAGES * F32_STAGE + TSTAGES * TERM_STAGE + SUM_BYTES + BAR_BYTES + 1024;
-};
-// kind::f16, BF16 x BF16 -> F32, K-major A and B, M = 256 (cta pair), N = 256
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
-                           ((uint32_t)(256 >> 4) << 24);
-}  // namespace t2
-
-struct T2Args {
-  GemmArgs g;
-  float* partial;                  // [(tiles - F) * S][256][256]
-  int TM, TN, NKT, tiles, F, ksplit, units, S;   // all below 2^31 (checked on the host)
-  int64_t c_max, p_max;            // largest element offset of C and of the partials (self-check)
-};
-
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -1142,6 +746,539 @@ __device__ __forceinline__ bool mbar_wait_cl(uint64_t* bar, uint32_t parity, vol
     }
   }
 }
+__device__ __forceinline__ float lds32(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+// The same with release at cluster scope.
+__device__ __forceinline__ void mbar_arrive_remote_cl(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+// Arrive (once) on the barrier at this shared-memory offset in the CTAs of
+// `mask` when every tcgen05.mma this thread issued so far has completed.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(mask)
+      : "memory");
+}
+template <int NT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
+    k_gemm_packed(const __grid_constant__ PkArgs t) {
+  using namespace pk;
+  constexpr int STAGES = Cfg<NT>::STAGES, STAGE_BYTES = Cfg<NT>::STAGE_BYTES, BLOB = Cfg<NT>::BLOB;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* peer_full = full + STAGES;     // (leader) the peer's stage has landed
+  uint64_t* empty = peer_full + STAGES;
+  uint64_t* chunk_done = empty + STAGES;
+  uint64_t* drained = chunk_done + 1;      // (leader) both CTAs' warps have drained the main accumulator
+  uint64_t* xdrained = drained + 1;        // (leader) and the cross accumulator
+  uint64_t* final_bar = xdrained + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const GemmArgs& g = t.g;
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_rank();
+  const int64_t cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&peer_full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(chunk_done, 1);
+    mbar_init(drained, 2 * NDRAIN / 32);
+    mbar_init(xdrained, 2 * NDRAIN / 32);
+    mbar_init(final_bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  cluster_sync_all();   // both CTAs' barriers initialised and TMEM allocated
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem_main = tmem, tmem_cross = tmem + 256;
+  const uint32_t sbase = smem_u32(smem);
+
+  // unit u -> tile (l, mt, nt; mt fastest), k-step range, split slot (-1: whole)
+  auto decode = [&](int64_t u, int64_t& l, int64_t& mt, int64_t& nt, int64_t& kb, int64_t& ke, int64_t& slot) {
+    int64_t tile;
+    if (u < t.F) {
+      tile = u; kb = 0; ke = t.NKT; slot = -1;
+    } else {
+      const int64_t v = u - t.F;
+      tile = t.F + v / t.S;
+      kb = (v % t.S) * t.ksplit;
+      ke = min(t.NKT, kb + t.ksplit);
+      slot = v;
+    }
+    mt = tile % t.TM;
+    const int64_t r = tile / t.TM;
+    nt = r % t.TN;
+    l = r / t.TN;
+  };
+
+  if (warp == 8) {
+    // ---------------- producer: this CTA's copies of a stage ----------------
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int64_t u = cid; u < t.units && ok; u += ncl) {
+        int64_t l, mt, nt, kb, ke, slot;
+        decode(u, l, mt, nt, kb, ke, slot);
+        // (a last odd tile stands in for the missing one: its rows or columns are not stored)
+        const int64_t ra = min(2 * mt + (int64_t)rank, t.RA - 1), rb = min(2 * nt + (int64_t)rank, t.RB - 1);
+        const unsigned char* pa = t.PA + ((l * t.RA + ra) * t.NKT) * (int64_t)BLOB;
+        const unsigned char* pb = t.PB + ((l * t.RB + rb) * t.NKT) * (int64_t)BLOB;
+        for (int64_t kt = kb; kt < ke; ++kt, ++it) {
+          const int s = it % STAGES;
+          if (it >= (uint32_t)STAGES && !mbar_wait_cl(&empty[s], ((it / STAGES) - 1) & 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&full[s], STAGE_BYTES);
+          const uint32_t d = sbase + s * STAGE_BYTES;
+          bulk_g2s(d, pa + kt * BLOB, BLOB, &full[s]);
+          bulk_g2s(d + BLOB, pb + kt * BLOB, BLOB, &full[s]);
+        }
+      }
+      // the copies of the last STAGES issues must land before the block exits
+      for (uint32_t i = it > (uint32_t)STAGES ? it - STAGES : 0; i < it; ++i)
+        mbar_wait_quiesce(&full[i % STAGES], (i / STAGES) & 1);
+    }
+  } else if (warp == 9) {
+    if (rank == 1 && lane == 0) {
+      // ---------------- peer: a landed stage, told to the leader ----------------
+      const uint32_t lead_full = peer_addr(smem_u32(peer_full), 0);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int64_t u = cid; u < t.units && ok; u += ncl) {
+        int64_t l, mt, nt, kb, ke, slot;
+        decode(u, l, mt, nt, kb, ke, slot);
+        for (int64_t kt = kb; kt < ke; ++kt, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&full[s], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+          mbar_arrive_remote_cl(lead_full + 8 * s);
+        }
+      }
+    } else if (rank == 0) {
+      // ---------------- leader: MMA issue ----------------
+      // the whole warp walks the stages (its descriptors stay in uniform
+      // registers), one elected lane issues
+      uint32_t it = 0, gc = 0, xc = 0;
+      bool ok = true;
+      for (int64_t u = cid; u < t.units && ok; u += ncl) {
+        int64_t l, mt, nt, kb, ke, slot;
+        decode(u, l, mt, nt, kb, ke, slot);
+        const int nk = (int)(ke - kb);
+        for (int j = 0; j < nk; ++j, ++it) {
+          const bool first = j % CHUNK == 0, xfirst = j % XCHUNK == 0;
+          const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
+          bool in = true;
+          if (xfirst && xc >= 1) in = mbar_wait_cl(xdrained, (xc - 1) & 1, abort_flag);
+          in = in && mbar_wait(&full[s], par, abort_flag) && mbar_wait_cl(&peer_full[s], par, abort_flag);
+          if (!__all_sync(0xffffffffu, in)) { ok = false; break; }
+          tc_fence_after();
+          const bool last = j % CHUNK == CHUNK - 1 || j == nk - 1;
+          const uint32_t sa = sbase + s * STAGE_BYTES, sb = sa + BLOB;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              bool start = xfirst && kk == 0;
+#pragma unroll
+              for (int d = 1; d < NT; ++d)
+#pragma unroll
+                for (int i = 0; i <= d; ++i) {
+                  umma_bf16_pair(tmem_cross, umma_desc(sa + i * TILE_BYTES + kk * 256),
+                                 umma_desc(sb + (d - i) * TILE_BYTES + kk * 256), start ? 0u : 1u, IDESC);
+                  start = false;
+                }
+            }
+          }
+          __syncwarp();
+          if (first && gc >= 1) {
+            in = mbar_wait_cl(drained, (gc - 1) & 1, abort_flag);
+            if (!__all_sync(0xffffffffu, in)) { ok = false; break; }
+            tc_fence_after();
+          }
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)
+              umma_bf16_pair(tmem_main, umma_desc(sa + kk * 256), umma_desc(sb + kk * 256),
+                             first && kk == 0 ? 0u : 1u, IDESC);
+            umma_commit_pair(&empty[s], 3);
+            if (last) umma_commit_pair(chunk_done, 3);
+          }
+          __syncwarp();
+          if (last) ++gc;
+          if (j % XCHUNK == XCHUNK - 1 || j == nk - 1) ++xc;
+        }
+      }
+      // every MMA this warp issued must finish before TMEM is freed, and the
+      // peer's arrivals must have landed before this CTA's shared memory goes
+      // (the commits track the MMAs of the lane that issued them)
+      if (elect_one()) {
+        umma_commit_pair(final_bar, 1);
+        mbar_wait_quiesce(final_bar, 0);
+        if (gc >= 1) mbar_wait_quiesce(drained, (gc - 1) & 1);
+        if (xc >= 1) mbar_wait_quiesce(xdrained, (xc - 1) & 1);
+      }
+      __syncwarp();
+    }
+  } else {
+    // ---------------- drain + epilogue (warps 0-7) ----------------
+    const int q = warp & 3, h = warp >> 2;
+    const int row = 32 * q + lane;
+    const int col0 = 128 * h;
+    const uint32_t lane_off = (uint32_t)(32 * q) << 16;
+    const uint32_t lead_drained = peer_addr(smem_u32(drained), 0), lead_xdrained = peer_addr(smem_u32(xdrained), 0);
+    uint32_t gc = 0, it = 0;
+    const float sx = scalar_as<float>(g.sx), sy = scalar_as<float>(g.sy);
+    float* Cp = static_cast<float*>(g.C);
+    for (int64_t u = cid; u < t.units; u += ncl) {
+      int64_t l, mt, nt, kb, ke, slot;
+      decode(u, l, mt, nt, kb, ke, slot);
+      const int nch = (int)((ke - kb + CHUNK - 1) / CHUNK);
+      it += (uint32_t)(ke - kb);
+      float sum[128];
+#pragma unroll
+      for (int j = 0; j < 128; ++j) sum[j] = 0.f;
+      bool ok = true;
+      auto drain = [&](uint32_t acc, uint32_t done) {   // one accumulator into the running sums
+#pragma unroll
+        for (int hh = 0; hh < 4; ++hh) {
+          uint32_t r[32];
+          __syncwarp();
+          tmem_ld32(acc + lane_off + (uint32_t)(col0 + 32 * hh), r);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[32 * hh + j] += __uint_as_float(r[j]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(done);
+      };
+      for (int ci = 0; ci < nch; ++ci, ++gc) {
+        if (!__all_sync(0xffffffffu, mbar_wait_cl(chunk_done, gc & 1, abort_flag))) { ok = false; break; }
+        tc_fence_after();
+        drain(tmem_main, lead_drained);
+        if (ci % (XCHUNK / CHUNK) == XCHUNK / CHUNK - 1 || ci == nch - 1) drain(tmem_cross, lead_xdrained);
+      }
+      if (!ok) break;
+      if (slot >= 0) {
+        float* pp = t.partial + (slot * 256 + col0) * (int64_t)256 + rank * BM + row;
+#pragma unroll
+        for (int j = 0; j < 128; ++j) pp[(int64_t)j * 256] = sum[j];
+      } else {
+        const int64_t m = mt * 256 + rank * BM + row;
+        if (m < g.M) {
+          const int64_t base = mode_offset(l, g.nl, g.l_ext, g.l_sc) + c_moff(g, m);
+          const int64_t n0 = nt * 256 + col0;
+          // 32 columns at a time through this thread's own shared memory, so
+          // that one short loop stores them all: 128 stores unrolled from the
+          // registers were fetched from memory once per tile, 70 us of them
+          const uint32_t mine = smem_u32(smem) + STAGES * STAGE_BYTES + 256 + 4 * tid;
+#pragma unroll 1
+          for (int pc = 0; pc < 4; ++pc) {
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+              if (pc == z)
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sts32(mine + j * (NDRAIN * 4), sum[32 * z + j]);
+#pragma unroll 2
+            for (int j = 0; j < 32; ++j) {
+              const int64_t n = n0 + 32 * pc + j;
+              if (n >= g.N) break;
+              float* cp = Cp + base + c_noff(g, n);
+              float o = lds32(mine + j * (NDRAIN * 4));
+              o = g.sx_one ? o : sx * o;
+              if (!g.sy_zero) o = fmaf(sy, *cp, o);
+              *cp = o;
+            }
+          }
+        }
+      }
+    }
+    // the leader's commits that free the last stages arrive on this CTA's
+    // barriers: wait for them before its shared memory can be reassigned
+    if (tid == 0)
+      for (uint32_t i = it > (uint32_t)STAGES ? it - STAGES : 0; i < it; ++i)
+        mbar_wait_quiesce(&empty[i % STAGES], (i / STAGES) & 1);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // the peer's drains and the leader's MMAs are over
+  if (warp == 9) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(pk::TMEM_COLS) : "memory");
+  }
+}
+
+// Sum the S split partials of each split tile in split order; αβ epilogue.  A
+// block takes four columns of a tile, a thread four rows of one (the partials
+// are read as 16-byte vectors, the splits' loads issued together).
+__global__ void __launch_bounds__(256) k_splitk_tiles(const __grid_constant__ PkArgs t) {
+  const GemmArgs& g = t.g;
+  const float sx = scalar_as<float>(g.sx), sy = scalar_as<float>(g.sy);
+  float* Cp = static_cast<float*>(g.C);
+  const int mloc = (threadIdx.x & 63) * 4;
+  const int64_t units = (t.tiles - t.F) * 64;
+  for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    const int64_t v = u >> 6;
+    const int nloc = (int)(u & 63) * 4 + (threadIdx.x >> 6);
+    const int64_t tile = t.F + v;
+    const int64_t mt = tile % t.TM, r2 = tile / t.TM, nt = r2 % t.TN, l = r2 / t.TN;
+    const int64_t m = mt * 256 + mloc, n = nt * 256 + nloc;
+    if (m >= g.M || n >= g.N) continue;
+    const float4* p = reinterpret_cast<const float4*>(t.partial + (v * t.S * 256 + nloc) * 256 + mloc);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int s = 0; s < t.S; ++s) {
+      const float4 w = p[(int64_t)s * (256 * 256 / 4)];
+      acc.x += w.x;
+      acc.y += w.y;
+      acc.z += w.z;
+      acc.w += w.w;
+    }
+    float* cn = Cp + mode_offset(l, g.nl, g.l_ext, g.l_sc) + c_noff(g, n);
+    const float f[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (m + i >= g.M) break;
+      float* cp = cn + c_moff(g, m + i);
+      float o = g.sx_one ? f[i] : sx * f[i];
+      if (!g.sy_zero) o = fmaf(sy, *cp, o);
+      *cp = o;
+    }
+  }
+}
+
+static void pack_args(PackArgs& p, const float* X, unsigned char* P, int64_t R, int nr, const int64_t* r_ext,
+                      const int64_t* r_str, const GemmArgs& g, const int64_t* k_str, const int64_t* l_str) {
+  memset(&p, 0, sizeof(p));
+  p.X = X;
+  p.P = P;
+  p.R = R;
+  p.K = g.K;
+  p.L = g.L;
+  p.RT = (R + pk::BM - 1) / pk::BM;
+  p.NKT = (g.K + pk::BK - 1) / pk::BK;
+  p.nr = nr;
+  p.nk = g.nk;
+  p.nl = g.nl;
+  for (int i = 0; i < nr; ++i) { p.r_ext[i] = r_ext[i]; p.r_str[i] = r_str[i]; }
+  for (int i = 0; i < g.nk; ++i) { p.k_ext[i] = g.k_ext[i]; p.k_str[i] = k_str[i]; }
+  for (int i = 0; i < g.nl; ++i) { p.l_ext[i] = g.l_ext[i]; p.l_str[i] = l_str[i]; }
+  p.kfast = k_str[0] == 1 && g.k_ext[0] % 8 == 0;
+}
+
+size_t gemm_packed_bytes(const GemmArgs& g, int nterms, int num_sms) {
+  using namespace pk;
+  const int64_t TM = (g.M + BM - 1) / BM, TN = (g.N + BM - 1) / BM, NKT = (g.K + BK - 1) / BK;
+  const size_t blob = (size_t)nterms * TILE_BYTES;
+  // packed operands + at most one grid's worth of split partials
+  return (size_t)g.L * (TM + TN) * NKT * blob + (size_t)(num_sms / 2) * 256 * 256 * 4 + 1024;
+}
+
+// The same product with the operands' roles exchanged.
+static GemmArgs gemm_swapped(const GemmArgs& q) {
+  GemmArgs g = q;
+  g.A = q.B; g.B = q.A;
+  g.M = q.N; g.N = q.M;
+  g.nm = q.nn; g.nn = q.nm;
+  for (int i = 0; i < MAXG; ++i) {
+    g.m_ext[i] = q.n_ext[i]; g.m_sa[i] = q.n_sb[i]; g.m_sc[i] = q.n_sc[i];
+    g.n_ext[i] = q.m_ext[i]; g.n_sb[i] = q.m_sa[i]; g.n_sc[i] = q.m_sc[i];
+    g.k_sa[i] = q.k_sb[i]; g.k_sb[i] = q.k_sa[i];
+    g.l_sa[i] = q.l_sb[i]; g.l_sb[i] = q.l_sa[i];
+  }
+  g.a_m_fast = q.b_n_fast; g.b_n_fast = q.a_m_fast;
+  return g;
+}
+
+cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, size_t ws_bytes, int num_sms,
+                               cudaStream_t s, int64_t* ctab) {
+  using namespace pk;
+  // consecutive threads store consecutive rows: the rows are the side that has
+  // C's contiguous mode
+  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;
+  if (!gemm_split_supported(g) || (nterms != 2 && nterms != 3)) return cudaErrorNotSupported;
+  static std::atomic<unsigned long long> attr2{0}, attr3{0};
+  {
+    const cudaError_t e = nterms == 2 ? set_smem_once(attr2, k_gemm_packed<2>, Cfg<2>::SMEM_BYTES)
+                                      : set_smem_once(attr3, k_gemm_packed<3>, Cfg<3>::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+  }
+  const int64_t TM = (g.M + BM - 1) / BM, TN = (g.N + BM - 1) / BM, NKT = (g.K + BK - 1) / BK;
+  const size_t blob = (size_t)nterms * TILE_BYTES;
+  const size_t bytes_a = (size_t)g.L * TM * NKT * blob, bytes_b = (size_t)g.L * TN * NKT * blob;
+  const int64_t TM2 = (TM + 1) / 2, TN2 = (TN + 1) / 2;   // 256 x 256 tiles of the CTA pairs
+  const int64_t tiles = g.L * TM2 * TN2;
+  const int64_t G = std::max(1, num_sms / 2);     // clusters
+  // whole tiles for every complete wave; the rest split along K so that the
+  // last wave covers the grid (at least 8 k-steps per split)
+  int64_t F = tiles >= G ? (tiles / G) * G : 0;
+  int64_t Rt = tiles - F;
+  int64_t S = 1;
+  if (Rt > 0) {
+    S = std::max<int64_t>(1, G / Rt);
+    S = std::min<int64_t>(S, std::max<int64_t>(1, NKT / 8));
+  }
+  const int64_t ksplit = (NKT + S - 1) / S;
+  S = (NKT + ksplit - 1) / ksplit;
+  if (S == 1) {
+    F = tiles;
+    Rt = 0;
+  }
+  const size_t bytes_p = (size_t)Rt * S * 256 * 256 * 4;
+  if (bytes_a + bytes_b + bytes_p + 768 > ws_bytes) return cudaErrorNotSupported;
+  unsigned char* w = static_cast<unsigned char*>(workspace);
+  unsigned char* PA = w;
+  unsigned char* PB = w + ((bytes_a + 255) & ~(size_t)255);
+  float* part = reinterpret_cast<float*>(PB + ((bytes_b + 255) & ~(size_t)255));
+
+  PackArgs pa, pb;
+  pack_args(pa, static_cast<const float*>(g.A), PA, g.M, g.nm, g.m_ext, g.m_sa, g, g.k_sa, g.l_sa);
+  pack_args(pb, static_cast<const float*>(g.B), PB, g.N, g.nn, g.n_ext, g.n_sb, g, g.k_sb, g.l_sb);
+  if (ctab) {
+    pa.c_tab = ctab;
+    pb.c_tab = ctab + g.M;
+    for (int i = 0; i < g.nm; ++i) pa.c_str[i] = g.m_sc[i];
+    for (int i = 0; i < g.nn; ++i) pb.c_str[i] = g.n_sc[i];
+  }
+  const int64_t units = g.L * (TM + TN) * NKT + (ctab ? (g.M + 255) / 256 + (g.N + 255) / 256 : 0);
+  const unsigned gp = (unsigned)std::min<int64_t>(units, (int64_t)num_sms * 8);
+  if (nterms == 2) k_pack_split<2><<<gp, 256, 0, s>>>(pa, pb);
+  else k_pack_split<3><<<gp, 256, 0, s>>>(pa, pb);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+
+  PkArgs t;
+  memset(&t, 0, sizeof(t));
+  t.g = g;
+  if (ctab) {
+    t.g.m_tab_c = ctab;
+    t.g.n_tab_c = ctab + g.M;
+  }
+  t.PA = PA;
+  t.PB = PB;
+  t.partial = part;
+  t.RA = TM;
+  t.RB = TN;
+  t.TM = TM2;
+  t.TN = TN2;
+  t.NKT = NKT;
+  t.tiles = tiles;
+  t.F = F;
+  t.S = (int)S;
+  t.ksplit = ksplit;
+  t.units = F + Rt * S;
+  const unsigned grid = (unsigned)(2 * std::min<int64_t>(t.units, G));
+  // plain launches: a GEMM block started early would hold its SM's shared
+  // memory and TMEM while waiting, which stalls other streams' kernels
+  {
+    KernelTimer kt(s, "k_gemm_packed");
+    if (nterms == 2) k_gemm_packed<2><<<grid, NTHREADS, Cfg<2>::SMEM_BYTES, s>>>(t);
+    else k_gemm_packed<3><<<grid, NTHREADS, Cfg<3>::SMEM_BYTES, s>>>(t);
+  }
+  count_launch();
+  e = cudaGetLastError();
+  if (e != cudaSuccess || Rt == 0) return e;
+  k_splitk_tiles<<<(unsigned)std::min<int64_t>(Rt * 64, (int64_t)num_sms * 16), 256, 0, s>>>(t);
+  count_launch();
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// k_gemm_tma2: 2-SM tensor-core GEMM fed by tensor maps over the FP32 inputs.
+//
+// The operands are read in place, through TMA tensor maps whose dimensions
+// and strides are the contraction's merged mode groups (the permutation of
+// simplifyto, src/einsum.jl:127-134, lives in the maps: nothing is written
+// back to HBM), and split into BF16 terms in shared memory.
+//  * A cluster of two CTAs computes a 256 x 256 tile of C with
+//    tcgen05.mma.cta_group::2 (M = 256, N = 256, K = 16): CTA r holds rows
+//    128r..128r+127 of the A tile and columns 128r..128r+127 of the B tile;
+//    its TMEM receives rows 128r.. of the accumulator, all 256 columns.
+//  * Warp 16 (one thread) issues, per 32-wide k stage, the TMA loads of this
+//    CTA's FP32 A and B tiles (128-byte swizzle, zero fill past the extents;
+//    no multicast) into one of three FP32 stages.
+//  * Warps 0-7 (A) and 8-15 (B) convert a stage into NT BF16 terms per value
+//    in the UMMA K-major canonical layout (conflict-free shared-memory reads
+//    and writes in both operand orientations), then arrive on the leader
+//    CTA's term_full barrier (remote arrive, release at cluster scope).
+//  * Warp 17 of the leader CTA issues the MMAs (main t0*t0 and cross-term
+//    accumulators, 2 x 256 TMEM columns) and releases each term stage to both
+//    CTAs with a multicast tcgen05.commit.
+//  * Every CHS stages the 16 converter warps of both CTAs drain the
+//    accumulators (tcgen05.ld) into FP32 running sums in registers with
+//    round-to-nearest adds; the accumulators are single-buffered, so the
+//    converters drain chunk c before they wait for a term stage whose MMAs
+//    come after it (no cycle in the waits).
+//  * Persistent over units: whole 256 x 256 tiles for the complete waves of
+//    clusters, the last wave's tiles cut along K (partials summed in split
+//    order by k_splitk_tiles2: deterministic).
+//  * Every wait is bounded (tc::WAIT_NS); on expiry the CTA records the
+//    timeout flag, stops waiting, lets its own copies and MMAs finish and
+//    frees its TMEM.  Both CTAs meet at a final cluster barrier.
+namespace t2 {
+constexpr int BM = 128;                    // rows per CTA (256 per cluster tile)
+constexpr int BK = 32;                     // k per stage
+constexpr int CHS = 8;                     // stages per accumulator chunk (16 k-steps)
+constexpr int F32_STAGES = 2;
+constexpr int NSR = 32;                    // running sums per thread in registers (the other NSR in shared memory)
+constexpr int F32_TILE = BM * BK * 4;      // 16 KB: one operand, one stage
+constexpr int TERM_TILE = BM * BK * 2;     // 8 KB: one term of one operand
+constexpr int NCONV = 512;                 // converter + drain warps 0-15
+constexpr int NTHREADS = NCONV + 64;       // + TMA warp 16 + MMA warp 17
+constexpr int TMEM_COLS = 512;
+template <int NT> struct Cfg {
+  static constexpr int F32_STAGE = 2 * F32_TILE;          // A tile, B tile
+  static constexpr int TERM_STAGE = 2 * NT * TERM_TILE;   // A terms, B terms
+  static constexpr int TSTAGES = NT == 2 ? 3 : 2;
+  static constexpr int SUM_BYTES = NCONV * (64 - NSR) * 4;   // 64 KB of running sums
+  static constexpr int BAR_BYTES = 256;
+  static constexpr int SMEM_BYTES = F32_STAGES * F32_STAGE + TSTAGES * TERM_STAGE + SUM_BYTES + BAR_BYTES + 1024;
+};
+// kind::f16, BF16 x BF16 -> F32, K-major A and B, M = 256 (cta pair), N = 256
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
+                           ((uint32_t)(256 >> 4) << 24);
+}  // namespace t2
+
+struct T2Args {
+  GemmArgs g;
+  float* partial;                  // [(tiles - F) * S][256][256]
+  int TM, TN, NKT, tiles, F, ksplit, units, S;   // all below 2^31 (checked on the host)
+  int64_t c_max, p_max;            // largest element offset of C and of the partials (self-check)
+};
+
 // 32-bit shared-address forms (fewer registers than generic pointers).
 __device__ __forceinline__ bool mbar_try_wait32(uint32_t a, uint32_t parity) {
   uint32_t ok;
@@ -1177,14 +1314,6 @@ __device__ __forceinline__ bool mbar_wait32(uint32_t a, uint32_t parity, uint32_
 __device__ __forceinline__ void mbar_arrive32(uint32_t a) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
 }
-__device__ __forceinline__ float lds32(uint32_t a) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ void sts32(uint32_t a, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
@@ -1197,22 +1326,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
       "[%5];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(t2::IDESC), "r"(acc));
-}
-// Arrive (once) on the barrier at this shared-memory offset in the CTAs of
-// `mask` when every tcgen05.mma this thread issued so far has completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(mask)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
@@ -1451,13 +1564,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(t2::NTHREADS, 1)
               bd[q] = umma_desc(sb + q * TERM_TILE + off);
             }
             const uint32_t keep = (first && kk == 0) ? 0u : 1u;
-            umma_bf16_pair(tmem_main, ad[0], bd[0], keep);
+            umma_bf16_pair(tmem_main, ad[0], bd[0], keep, IDESC);
             bool first_cross = true;
 #pragma unroll
             for (int d = 1; d < NT; ++d)
 #pragma unroll
               for (int i = 0; i <= d; ++i) {
-                umma_bf16_pair(tmem_cross, ad[i], bd[d - i], first_cross ? keep : 1u);
+                umma_bf16_pair(tmem_cross, ad[i], bd[d - i], first_cross ? keep : 1u, IDESC);
                 first_cross = false;
               }
           }
@@ -1556,11 +1669,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(t2::NTHREADS, 1)
             float* crow = static_cast<float*>(g.C) + roff;
             const int64_t nsc = g.n_sc[0];
             const int n0 = dnt * 256 + col0;
+            // one short loop stores the columns held in shared memory, then,
+            // through the same places, those held in registers (64 unrolled
+            // stores with their checks were fetched from memory once per tile)
+#pragma unroll 1
+            for (int half = 1; half >= 0; --half) {
+              if (half == 0)
 #pragma unroll
-            for (int j = 0; j < 64; ++j) {
-              if (n0 + j < g.N && in_bounds(roff + (int64_t)(n0 + j) * nsc, t.c_max, 1)) {
-                float* cp = crow + (int64_t)(n0 + j) * nsc;
-                const float v = j < NSR ? sum[j] : lds32(ssum + (uint32_t)((j - NSR) * NCONV * 4));
+                for (int j = 0; j < NSR; ++j) sts32(ssum + (uint32_t)(j * NCONV * 4), sum[j]);
+#pragma unroll 2
+              for (int j = 0; j < NSR; ++j) {
+                const int n = n0 + half * NSR + j;
+                if (n >= g.N || !in_bounds(roff + (int64_t)n * nsc, t.c_max, 1)) break;
+                float* cp = crow + (int64_t)n * nsc;
+                const float v = lds32(ssum + (uint32_t)(j * NCONV * 4));
                 float o = g.sx_one ? v : sx * v;
                 if (!g.sy_zero) o = fmaf(sy, *cp, o);
                 *cp = o;
@@ -1732,8 +1854,9 @@ size_t gemm_tma2_bytes(const GemmArgs& g, int num_sms) {
   return (size_t)(num_sms / 2) * 256 * 256 * 4 + 1024;
 }
 
-cudaError_t launch_gemm_tma2(const GemmArgs& g, int nterms, void* workspace, size_t ws_bytes, int num_sms,
+cudaError_t launch_gemm_tma2(const GemmArgs& q, int nterms, void* workspace, size_t ws_bytes, int num_sms,
                              cudaStream_t s) {
+  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;   // (as in launch_gemm_packed)
   if ((nterms != 2 && nterms != 3) || !gemm_tma2_applies(g)) return cudaErrorNotSupported;
   const bool ak = g.k_sa[0] == 1, bk = g.k_sb[0] == 1;
   alignas(64) CUtensorMap ma, mb;

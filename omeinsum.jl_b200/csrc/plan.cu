@@ -488,7 +488,7 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
       }
     if (M < 256 || N < 256 || K < 512 || 2.0 * M * N * K * L < 1e9) return 0;
     const double bytes = L * (std::ceil(M / 128) + std::ceil(N / 128)) * std::ceil(K / 32) * 3 * 8192 +
-                         148.0 * 128 * 128 * 4 + (M + N) * 8 + 4096;
+                         74.0 * 256 * 256 * 4 + (M + N) * 8 + 4096;
     return bytes <= (double)((size_t)2 << 30) ? (size_t)bytes : 0;
   };
   auto scratch_bound = [&](bool use_sliced) {
