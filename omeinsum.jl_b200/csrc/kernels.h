@@ -124,6 +124,7 @@ struct TinyNode {
   const void* x0;
   const void* x1;       // NULL: one input
   void* y;
+  void* yw;             // the result in the sums' type too (NULL: only in y)
   uint32_t n_out, n_in;
   uint32_t item0;       // first warp item of the node in its level
   uint8_t nout, ninner; // modes [0, nout) are output modes, then the summed ones
@@ -131,12 +132,15 @@ struct TinyNode {
   uint8_t pad;
   alignas(16) TinyMode mode[TINY_MODES];
 };
-enum TinyFlags { TINY_CONJ0 = 1, TINY_CONJ1 = 2, TINY_CONJY = 4, TINY_WARP = 8 };
+// TINY_WIDE*: the operand is a node's result in the sums' type.
+enum TinyFlags { TINY_CONJ0 = 1, TINY_CONJ1 = 2, TINY_CONJY = 4, TINY_WARP = 8, TINY_WIDE0 = 16, TINY_WIDE1 = 32 };
+// Bytes per element of the type that sums run in (Float64 for Float32).
+size_t tiny_wide_size(ome_dtype dt);
 // The node's contraction of labelled views (data pointers are not used); false
 // if it does not fit a TinyNode.
 struct HView;
 bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y);
-// Runs nodes[0..n) (level[i] ascending); one launch per 104 nodes.
+// Runs nodes[0..n) (level[i] ascending); one launch per 100 nodes.
 cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, cudaStream_t s);
 
 // Read and clear the CUDA-core GEMM's split-partial self-check flag.

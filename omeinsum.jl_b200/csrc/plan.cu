@@ -36,6 +36,9 @@ struct PNode {
   size_t off_fwd = 0;              // workspace offset in sliced forward
   size_t off_keep = 0;             // offset of the forward value when all are kept
   size_t off_grad = 0;             // offset of the gradient buffer
+  // offsets of the same in the tiny programs' wider type (tiny nodes only)
+  size_t off_fwd_w = 0, off_keep_w = 0, off_grad_w = 0;
+  bool grad_tiny = false;          // the gradient is written by the reverse program
   int parent = -1;
   bool tiny = false;               // (sliced sizes) the node and its whole subtree are small contractions
   bool tiny_full = false;          // the same with full sizes
@@ -77,6 +80,7 @@ struct ome_plan {
   size_t arena_bytes = 0, grad_arena = 0;  // planned buffers (forward / gradient)
   size_t fwd_bytes = 0, grad_bytes = 0;     // plus per-node dispatch scratch
   size_t esize = 0;
+  size_t wsize = 0;                // bytes of the wider type; 0 if it is the element type
   // steps of the tiny programs, levels ascending: forward on sliced and on
   // full sizes, reverse sweep; programs built for the last input strides seen
   // (several threads may evaluate one plan)
@@ -319,7 +323,10 @@ void plan_tiny(ome_plan* p) {
       s.kind[2] = r >= 0 ? TinyStep::GRAD : TinyStep::INPUT_GRAD;
       s.ref[2] = r >= 0 ? r : -r - 1;
       if (cplx) s.flags = TINY_CONJY | (i == 0 ? TINY_CONJ0 : TINY_CONJ1);
-      if (r >= 0) lev[r] = lev[j] + 1;
+      if (r >= 0) {
+        lev[r] = lev[j] + 1;
+        p->nodes[r].grad_tiny = true;
+      }
       p->steps[TINY_REV].push_back(s);
     }
   }
@@ -345,6 +352,7 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   p->dt = dtype;
   p->prec = prec;
   p->esize = dtype_size(dtype);
+  p->wsize = tiny_wide_size(dtype) == p->esize ? 0 : tiny_wide_size(dtype);
   p->ninputs = ninputs;
   for (int i = 0; i < nlabels; ++i) {
     if (label_extents[i] < 0) {
@@ -435,6 +443,12 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   if (p->acc64) p->acc_off = ar.alloc((size_t)p->nodes[root].numel * (dtype == OME_C32 ? 16 : 8));
   for (int j = 0; j < root; ++j)
     if (p->nodes[j].tiny) p->nodes[j].off_fwd = ar.alloc((size_t)p->nodes[j].numel_s * p->esize);
+  if (p->wsize) {   // (wide copies live through the program only)
+    for (int j = 0; j < root; ++j)
+      if (p->nodes[j].tiny) p->nodes[j].off_fwd_w = ar.alloc((size_t)p->nodes[j].numel_s * p->wsize);
+    for (int j = 0; j < root; ++j)
+      if (p->nodes[j].tiny) ar.release(p->nodes[j].off_fwd_w);
+  }
   for (int j = 0; j < root; ++j)
     if (p->nodes[j].tiny)
       for (int r : p->nodes[j].args)
@@ -524,6 +538,19 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
     n.off_grad = g;
     g += ((size_t)n.numel * p->esize + 255) & ~(size_t)255;
   }
+  if (p->wsize)
+    for (int j = 0; j < root; ++j) {
+      PNode& n = p->nodes[j];
+      const size_t b = ((size_t)n.numel * p->wsize + 255) & ~(size_t)255;
+      if (n.tiny_full) {
+        n.off_keep_w = g;
+        g += b;
+      }
+      if (n.grad_tiny) {
+        n.off_grad_w = g;
+        g += b;
+      }
+    }
   p->dy_off = g;
   p->grad_arena = g + ((size_t)p->nodes[root].numel * p->esize + 511);
   p->grad_bytes = ((p->grad_arena + 255) & ~(size_t)255) + scratch_grad;
@@ -650,9 +677,10 @@ std::shared_ptr<const TinyProgram> tiny_program(ome_plan* p, int which, const Le
 
 // Runs a tiny program; *done = false (nothing launched) if the input strides
 // do not fit its descriptors.  y: where a tree that is tiny as a whole puts
-// its value (NULL: the root is left out).
+// its value (NULL: the root is left out).  values_wide: the tiny nodes' values
+// are there in the wider type too.
 int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves& in, const std::vector<int64_t>& fix,
-             char* y, char* dy_root, void* const* dxs, bool* done) {
+             char* y, char* dy_root, void* const* dxs, bool values_wide, bool* done) {
   *done = true;
   const auto& steps = p->steps[which];
   if (steps.empty()) return OME_OK;
@@ -686,11 +714,24 @@ int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves&
   std::vector<TinyNode> nodes(prog->nodes);
   size_t count = steps.size();
   if (steps.back().kind[2] == TinyStep::OUTPUT && !y) --count;
+  // the wider copy of a value or gradient (NULL: there is none)
+  auto wide = [&](TinyStep::Kind k, int ref) -> char* {
+    if (!p->wsize || (k != TinyStep::VALUE && k != TinyStep::GRAD) || ref == root) return nullptr;
+    const PNode& n = p->nodes[ref];
+    if (k == TinyStep::VALUE && values_wide && (keep ? n.tiny_full : n.tiny)) return ctx->ws + (keep ? n.off_keep_w : n.off_fwd_w);
+    return k == TinyStep::GRAD && n.grad_tiny ? ctx->ws + n.off_grad_w : nullptr;
+  };
   for (size_t i = 0; i < count; ++i) {
     const TinyStep& st = steps[i];
-    nodes[i].x0 = at(st.kind[0], st.ref[0]);
-    nodes[i].x1 = st.nin > 1 ? at(st.kind[1], st.ref[1]) : nullptr;
-    nodes[i].y = at(st.kind[2], st.ref[2]);
+    TinyNode& n = nodes[i];
+    for (int a = 0; a < st.nin; ++a) {
+      char* w = wide(st.kind[a], st.ref[a]);
+      (a == 0 ? n.x0 : n.x1) = w ? w : at(st.kind[a], st.ref[a]);
+      if (w) n.flags |= a == 0 ? TINY_WIDE0 : TINY_WIDE1;
+    }
+    if (st.nin == 1) n.x1 = nullptr;
+    n.y = at(st.kind[2], st.ref[2]);
+    n.yw = wide(st.kind[2], st.ref[2]);
   }
   return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)count, s), "tiny program");
 }
@@ -699,14 +740,15 @@ int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves&
 // other nodes in post-order.  y: the tree's output if its value goes there as
 // it is; *rooted = true if the program has put it there.
 int run_forward(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves& inputs,
-                const std::vector<int64_t>& fix, size_t scratch, char* y, bool* rooted) {
+                const std::vector<int64_t>& fix, size_t scratch, char* y, bool* rooted, bool* programmed) {
   const bool sliced = which == TINY_FWD && !p->sliced.empty(), keep = which != TINY_FWD;
   static const std::vector<int32_t> none;
   static const std::vector<int64_t> nofix;
   const Scalar one = scalar_one(p->dt), zero = scalar_zero(p->dt);
   const int root = (int)p->nodes.size() - 1;
   bool done = false;
-  int rc = run_tiny(ctx, p, s, which, inputs, fix, y, nullptr, nullptr, &done);
+  int rc = run_tiny(ctx, p, s, which, inputs, fix, y, nullptr, nullptr, true, &done);
+  *programmed = done;
   if (rc) return rc;
   *rooted = done && y && !p->steps[which].empty() && p->steps[which].back().kind[2] == TinyStep::OUTPUT;
   auto one_node = [&](int j) {
@@ -746,8 +788,8 @@ int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, 
       fix[i] = r % ext;
       r /= ext;
     }
-    bool rooted;
-    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, fix, scratch, nullptr, &rooted);
+    bool rooted, programmed;
+    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, fix, scratch, nullptr, &rooted, &programmed);
     if (rc) return rc;
     if (p->acc64) {
       HView tv = make_view(p, ctx->ws + p->tmp_off, rn.iy_s, none, nofix);
@@ -796,9 +838,9 @@ int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void
   static const std::vector<int64_t> nofix;
 
   if (p->sliced.empty()) {
-    bool rooted;
+    bool rooted, programmed;
     const bool plain = scalar_is_one(dt, sx) && scalar_is_zero(dt, sy);
-    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, nofix, scratch, plain ? (char*)y : nullptr, &rooted);
+    int rc = run_forward(ctx, p, s, TINY_FWD, inputs, nofix, scratch, plain ? (char*)y : nullptr, &rooted, &programmed);
     if (rc || rooted) return rc;
     HView yv = make_view(p, (char*)y, rn.iy, none, nofix);
     return run_node(ctx, p, s, root, inputs, false, nofix, off_fwd_of, yv, sx, sy, scratch);
@@ -921,8 +963,8 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
   static const std::vector<int64_t> nofix;
   const size_t scratch = (p->grad_arena + 255) & ~(size_t)255;
   // forward, every value kept
-  bool rooted;
-  int rc = run_forward(ctx, p, s, TINY_FWD_FULL, inputs, nofix, scratch, (char*)y, &rooted);
+  bool rooted, programmed;
+  int rc = run_forward(ctx, p, s, TINY_FWD_FULL, inputs, nofix, scratch, (char*)y, &rooted, &programmed);
   if (rc) return rc;
   HView yv = make_view(p, (char*)y, rn.iy, none, nofix);
   if (!rooted) rc = run_node(ctx, p, s, root, inputs, false, nofix, off_keep_of, yv, one, zero, scratch);
@@ -985,7 +1027,7 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
       }
     }
   }
-  if (tiny) return run_tiny(ctx, p, s, TINY_REV, inputs, nofix, nullptr, dy_root, dxs, &tiny);
+  if (tiny) return run_tiny(ctx, p, s, TINY_REV, inputs, nofix, nullptr, dy_root, dxs, programmed, &tiny);
   return OME_OK;
 }
 

@@ -29,12 +29,14 @@ struct TinyArgs {
   uint32_t items[TINY_LEVELS];       // warp items of each level
   TinyNode nodes[CAP];
 };
-// 104 nodes are 32.0 KB of the 32764 bytes a launch's arguments may have
-constexpr int TINY_CAP = 104, TINY_CAP_SMALL = 12;
+// 100 nodes are 32.4 KB of the 32764 bytes a launch's arguments may have
+constexpr int TINY_CAP = 100, TINY_CAP_SMALL = 12;
 static_assert(sizeof(TinyArgs<TINY_CAP>) <= 32764, "kernel arguments");
 
 // Sums run in the type W: Float64 for Float32 elements, the element type
-// otherwise.
+// otherwise.  A result is kept in W too, for the nodes of the program that read
+// it: in a network of 160 vertices the roundings of the 144 small nodes to
+// Float32 were most of the value's error.
 template <class A> struct TinyWide { using W = A; };
 template <> struct TinyWide<AlgF32> { using W = AlgF64; };
 template <> struct TinyWide<AlgC32> { using W = AlgC64; };
@@ -110,18 +112,22 @@ __global__ void __launch_bounds__(TINY_THREADS) k_tiny(const __grid_constant__ T
         o0 += d * md.s0;
         o1 += d * md.s1;
       }
-      const T* x0 = static_cast<const T*>(n.x0) + o0;
-      const T* x1 = static_cast<const T*>(n.x1) + o1;
+      constexpr bool WIDE = !std::is_same<T, W>::value;
+      const bool w0 = WIDE && (n.flags & TINY_WIDE0), w1 = WIDE && (n.flags & TINY_WIDE1);
+      const T* x0 = static_cast<const T*>(n.x0) + (w0 ? 0 : o0);
+      const T* x1 = static_cast<const T*>(n.x1) + (w1 ? 0 : o1);
+      const W* x0w = static_cast<const W*>(n.x0) + (w0 ? o0 : 0);
+      const W* x1w = static_cast<const W*>(n.x1) + (w1 ? o1 : 0);
       const bool two = n.x1 != nullptr, c0 = n.flags & TINY_CONJ0, c1 = n.flags & TINY_CONJ1;
       W acc = WA::zero();
       const uint32_t step = by_warp ? 32u : 1u;
       // a single summed mode (the usual case) needs no decomposition
       const bool flat = n.ninner == 1;
       const int32_t f0 = flat ? n.mode[n.nout].s0 : 0, f1 = flat ? n.mode[n.nout].s1 : 0;
-      constexpr int U = sizeof(T) <= 8 ? 8 : 4;
+      constexpr int U = sizeof(W) <= 8 ? 8 : 4;
       for (uint32_t jb = by_warp ? lane : 0; jb < n.n_in; jb += U * step) {
         // U steps' loads, then their sums in order
-        T v0[U], v1[U];
+        W v0[U], v1[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           uint32_t j = jb + u * step;
@@ -136,22 +142,25 @@ __global__ void __launch_bounds__(TINY_THREADS) k_tiny(const __grid_constant__ T
                 i1 += d * md.s1;
               }
             }
-            v0[u] = tiny_ld(x0 + i0);
-            if (two) v1[u] = tiny_ld(x1 + i1);
+            v0[u] = w0 ? tiny_ld(x0w + i0) : tiny_as<W>(tiny_ld(x0 + i0));
+            if (two) v1[u] = w1 ? tiny_ld(x1w + i1) : tiny_as<W>(tiny_ld(x1 + i1));
           }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
           if (jb + u * step < n.n_in) {
-            W p = tiny_as<W>(tiny_conj(v0[u], c0));
-            if (two) p = WA::mul(p, tiny_as<W>(tiny_conj(v1[u], c1)));
+            W p = tiny_conj(v0[u], c0);
+            if (two) p = WA::mul(p, tiny_conj(v1[u], c1));
             acc = WA::add(acc, p);
           }
       }
       if (by_warp)
         for (int d = 16; d > 0; d >>= 1) acc = WA::add(acc, shfl_down_any(acc, d));
-      if (in && (!by_warp || lane == 0))
-        static_cast<T*>(n.y)[yo] = tiny_conj(tiny_as<T>(acc), n.flags & TINY_CONJY);
+      if (in && (!by_warp || lane == 0)) {
+        acc = tiny_conj(acc, n.flags & TINY_CONJY);
+        if (n.y) static_cast<T*>(n.y)[yo] = tiny_as<T>(acc);
+        if (WIDE && n.yw) static_cast<W*>(n.yw)[yo] = acc;
+      }
     }
     if (lev + 1 < a.nlevels) cl.sync();
   }
@@ -202,6 +211,12 @@ cudaError_t launch_tiny_t(const TinyNode* nodes, const int* level, int n, cudaSt
 }
 
 }  // namespace
+
+size_t tiny_wide_size(ome_dtype dt) {
+  size_t r = 0;
+  OME_DISPATCH(dt, ALG, r = sizeof(typename TinyWide<ALG>::W::T));
+  return r;
+}
 
 bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y) {
   if (nin < 1 || nin > 2) return false;
