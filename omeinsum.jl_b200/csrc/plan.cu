@@ -84,12 +84,20 @@ struct ome_plan {
   // steps of the tiny programs, levels ascending: forward on sliced and on
   // full sizes, reverse sweep; programs built for the last input strides seen
   // (several threads may evaluate one plan)
-  std::vector<TinyStep> steps[3];
-  std::shared_ptr<const TinyProgram> prog[3];
+  std::vector<TinyStep> steps[5];
+  std::shared_ptr<const TinyProgram> prog[5];
   std::mutex prog_mutex;
   std::vector<std::vector<char>> rev_tiny;   // [node][child]: the gradient step is in the reverse program
+  // Small Float32 / ComplexF32 trees are evaluated in Float64 / ComplexF64: the
+  // same tree planned in that type, and where its inputs, output, cotangent and
+  // gradients lie at the start of the workspace.
+  std::unique_ptr<ome_plan> wide;
+  std::vector<size_t> wide_in, wide_dx;
+  size_t wide_y = 0, wide_dy = 0, wide_base = 0;
 };
-enum { TINY_FWD = 0, TINY_FWD_FULL = 1, TINY_REV = 2 };
+// forward on sliced and on full sizes, reverse sweep, inputs to the wider type,
+// gradients from it
+enum { TINY_FWD = 0, TINY_FWD_FULL = 1, TINY_REV = 2, TINY_WIDEN = 3, TINY_NARROW = 4 };
 
 namespace {
 
@@ -334,6 +342,26 @@ void plan_tiny(ome_plan* p) {
                    [](const TinyStep& a, const TinyStep& b) { return a.level < b.level; });
 }
 
+// Multiply-adds of all nodes on full sizes.
+double plan_work(const ome_plan* p) {
+  double total = 0;
+  for (const PNode& n : p->nodes) {
+    std::vector<int32_t> seen;
+    double w = 1;
+    auto visit = [&](const std::vector<int32_t>& l) {
+      for (int32_t x : l)
+        if (!contains(seen, x)) {
+          seen.push_back(x);
+          w *= (double)p->ext.at(x);
+        }
+    };
+    visit(n.iy);
+    for (int r : n.args) visit(r >= 0 ? p->nodes[r].iy : p->in_labels[-r - 1]);
+    total += w;
+  }
+  return total;
+}
+
 }  // namespace
 
 extern "C" {
@@ -554,6 +582,52 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   p->dy_off = g;
   p->grad_arena = g + ((size_t)p->nodes[root].numel * p->esize + 511);
   p->grad_bytes = ((p->grad_arena + 255) & ~(size_t)255) + scratch_grad;
+  // Small trees in Float64: every value is then rounded to 32 bits once, at the
+  // end, where the roundings of a hundred nodes are amplified by the network's
+  // cancellations (a 100-vertex network's gradients 7e-7 off), and at this size
+  // (2^26 multiply-adds are 8 us of the FP64 pipe) the launches set the time
+  // (below eight nodes the two conversions' launches would be felt).
+  if ((dtype == OME_F32 || dtype == OME_C32) && prec != OME_PREC_FP32 && !sliced && nnodes >= 8 &&
+      plan_work(p) <= 0x1p26) {
+    bool small = true;
+    for (auto& l : p->in_labels) {
+      double n = 1;
+      for (int32_t x : l) n *= (double)p->ext[x];
+      small = small && n >= 1 && n <= (double)TINY_WORK && l.size() <= TINY_MODES;
+    }
+    ome_plan* w = nullptr;
+    const ome_dtype wt = dtype == OME_F32 ? OME_F64 : OME_C64;
+    if (small && ome_plan_create(ctx, wt, ninputs, input_nlabels, input_labels, nnodes, node_nargs, node_args, node_niy,
+                                 node_iy, nlabels, label_ids, label_extents, 0, nullptr, prec, &w) == OME_OK) {
+      p->wide.reset(w);
+      size_t at = 0;
+      auto take = [&](int64_t n) {
+        const size_t o = at;
+        at += ((size_t)std::max<int64_t>(n, 1) * w->esize + 255) & ~(size_t)255;
+        return o;
+      };
+      for (int grad = 0; grad < 2; ++grad)
+        for (auto& l : p->in_labels) {
+          int64_t n = 1;
+          for (int32_t x : l) n *= p->ext[x];
+          (grad ? p->wide_dx : p->wide_in).push_back(take(n));
+        }
+      p->wide_y = take(p->nodes[root].numel);
+      p->wide_dy = take(p->nodes[root].numel);
+      p->wide_base = at;
+      p->fwd_bytes = std::max(p->fwd_bytes, at + w->fwd_bytes);
+      p->grad_bytes = std::max(p->grad_bytes, at + w->grad_bytes);
+      for (int which : {TINY_WIDEN, TINY_NARROW})
+        for (int t = 0; t < ninputs; ++t) {
+          TinyStep st;
+          st.nin = 1;
+          st.kind[0] = TinyStep::INPUT;
+          st.kind[2] = TinyStep::INPUT_GRAD;
+          st.ref[0] = st.ref[2] = t;
+          p->steps[which].push_back(st);
+        }
+    }
+  }
   *out = p;
   return OME_OK;
 }
@@ -654,11 +728,16 @@ std::shared_ptr<const TinyProgram> tiny_program(ome_plan* p, int which, const Le
   const Leaves nowhere{null.data(), in.str};
   for (const TinyStep& st : p->steps[which]) {
     HView xs[2], y;
-    for (int a = 0; a < st.nin; ++a)
+    if (which >= TINY_WIDEN) {   // a copy, mode by mode (the labels may repeat)
+      xs[0] = which == TINY_WIDEN ? leaf_view(p, nowhere, st.ref[0], none, fix)
+                                  : make_view(p, nullptr, p->in_labels[st.ref[0]], none, fix);
+      y = make_view(p, nullptr, p->in_labels[st.ref[2]], none, fix);
+      for (int d = 0; d < y.nd; ++d) xs[0].lab[d] = y.lab[d] = d;
+    } else for (int a = 0; a < st.nin; ++a)
       xs[a] = st.kind[a] == TinyStep::INPUT
                   ? leaf_view(p, nowhere, st.ref[a], drop, fix)
                   : make_view(p, nullptr, sliced ? p->nodes[st.ref[a]].iy_s : p->nodes[st.ref[a]].iy, none, fix);
-    y = st.kind[2] == TinyStep::INPUT_GRAD
+    if (which < TINY_WIDEN) y = st.kind[2] == TinyStep::INPUT_GRAD
             ? make_view(p, nullptr, p->in_labels[st.ref[2]], none, fix)
             : make_view(p, nullptr, sliced ? p->nodes[st.ref[2]].iy_s : p->nodes[st.ref[2]].iy, none, fix);
     TinyNode n;
@@ -812,6 +891,37 @@ int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, 
   return OME_OK;
 }
 
+// The context above the wide plan's buffers.
+struct WideCtx {
+  ome_ctx* outer;
+  ome_ctx inner;
+  WideCtx(ome_ctx* c, const ome_plan* p) : outer(c), inner(*c) {
+    inner.ws += p->wide_base;
+    inner.ws_bytes -= p->wide_base;
+  }
+  ~WideCtx() {   // the overflow scratch may have grown
+    outer->ovf = inner.ovf;
+    outer->ovf_bytes = inner.ovf_bytes;
+  }
+};
+
+// The inputs in the wider type, at wide_in; *done = false if their strides do
+// not fit a program.
+int widen_inputs(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& in, std::vector<const void*>& out,
+                 bool* done) {
+  auto prog = tiny_program(p, TINY_WIDEN, in);
+  *done = prog->ok;
+  if (!prog->ok) return OME_OK;
+  std::vector<TinyNode> nodes(prog->nodes);
+  out.resize(p->ninputs);
+  for (int t = 0; t < p->ninputs; ++t) {
+    out[t] = ctx->ws + p->wide_in[t];
+    nodes[t].x0 = in.data[t];
+    nodes[t].yw = ctx->ws + p->wide_in[t];
+  }
+  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)nodes.size(), s), "inputs to Float64");
+}
+
 }  // namespace
 
 extern "C" {
@@ -830,6 +940,21 @@ int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const ome_dtype dt = p->dt;
   const Scalar sx = scalar_from(dt, sxp), sy = scalar_from(dt, syp);
+  if (p->wide) {
+    std::vector<const void*> win;
+    bool done;
+    int rc = widen_inputs(ctx, p, s, inputs, win, &done);
+    if (rc) return rc;
+    if (done) {
+      const ome_dtype wt = p->wide->dt;
+      const Scalar one = scalar_one(wt), zero = scalar_zero(wt);
+      WideCtx wc(ctx, p);
+      rc = ome_plan_execute(&wc.inner, p->wide.get(), stream, win.data(), ctx->ws + p->wide_y, one.b, zero.b);
+      if (rc) return rc;
+      return cuda_err(launch_acc64_store(dt, y, ctx->ws + p->wide_y, p->nodes.back().numel, sx, sy,
+                                         scalar_is_zero(dt, sy), s), "output from Float64");
+    }
+  }
   const Scalar one = scalar_one(dt), zero = scalar_zero(dt);
   const int root = (int)p->nodes.size() - 1;
   const PNode& rn = p->nodes[root];
@@ -897,6 +1022,8 @@ int ome_plan_execute_slices(ome_ctx* ctx, ome_plan* p, void* stream, const void*
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int root = (int)p->nodes.size() - 1;
   const PNode& rn = p->nodes[root];
+  if (p->wide && slice_end > slice_begin)   // (unsliced: the one slice is the whole tree)
+    return ome_plan_execute(ctx, p, stream, inputs, partial, scalar_one(p->dt).b, scalar_zero(p->dt).b);
   if (p->acc64) {
     const size_t w = p->dt == OME_C32 ? 16 : 8;
     int rc = cuda_err(cudaMemsetAsync(partial, 0, (size_t)rn.numel * w, s), "memset");
@@ -959,6 +1086,36 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
   const Scalar one = scalar_one(dt), zero = scalar_zero(dt);
   const int root = (int)p->nodes.size() - 1;
   const PNode& rn = p->nodes[root];
+  if (p->wide) {
+    std::vector<const void*> win;
+    bool done;
+    int rc = widen_inputs(ctx, p, s, inputs, win, &done);
+    if (rc) return rc;
+    if (done) {
+      if (dy) {
+        if (dt == OME_F32) rc = cuda_err(cudaMemsetAsync(ctx->ws + p->wide_dy, 0, (size_t)rn.numel * 8, s), "memset");
+        else rc = cuda_err(cudaMemsetAsync(ctx->ws + p->wide_dy, 0, (size_t)rn.numel * 16, s), "memset");
+        if (!rc) rc = cuda_err(launch_acc64(dt, ctx->ws + p->wide_dy, dy, rn.numel, s), "cotangent to Float64");
+        if (rc) return rc;
+      }
+      std::vector<void*> wdx(p->ninputs);
+      for (int t = 0; t < p->ninputs; ++t) wdx[t] = ctx->ws + p->wide_dx[t];
+      WideCtx wc(ctx, p);
+      rc = ome_plan_gradient(&wc.inner, p->wide.get(), stream, win.data(), dy ? ctx->ws + p->wide_dy : nullptr,
+                             ctx->ws + p->wide_y, wdx.data());
+      if (rc) return rc;
+      auto prog = tiny_program(p, TINY_NARROW, Leaves{nullptr, nullptr});
+      std::vector<TinyNode> nodes(prog->nodes);
+      for (int t = 0; t < p->ninputs; ++t) {
+        nodes[t].x0 = wdx[t];
+        nodes[t].flags |= TINY_WIDE0;
+        nodes[t].y = dxs[t];
+      }
+      rc = cuda_err(launch_tiny(dt, nodes.data(), prog->level.data(), (int)nodes.size(), s), "gradients from Float64");
+      if (rc) return rc;
+      return cuda_err(launch_acc64_store(dt, y, ctx->ws + p->wide_y, rn.numel, one, zero, 1, s), "output from Float64");
+    }
+  }
   static const std::vector<int32_t> none;
   static const std::vector<int64_t> nofix;
   const size_t scratch = (p->grad_arena + 255) & ~(size_t)255;
