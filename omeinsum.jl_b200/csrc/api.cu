@@ -690,6 +690,28 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       if (e != cudaErrorNotSupported) return cuda_err(e, "bf16 split gemm");
       cudaGetLastError();
     }
+    // Large ComplexF32 products on the tensor cores: real BF16x6 products of the
+    // 2 x 2 embedding (1024^3 259 us on the CUDA cores, 77 us here), whose error
+    // of 1.3e-7 .. 2e-7 lies below the CUDA cores' from K = 128 on
+    if (dt == OME_C32 && prec != OME_PREC_FP32 && M >= 128 && N >= 128 && K >= 128 && g.sx_one && g.sy_zero &&
+        8.0 * (double)M * (double)N * (double)K * (double)L >= 1e9) {
+      const size_t top = ctx->ws_top;
+      int64_t* tab = static_cast<int64_t*>(ws_alloc(ctx, (size_t)(2 * (M + N)) * sizeof(int64_t)));
+      size_t avail = ctx->ws_bytes > ctx->ws_top ? ctx->ws_bytes - ((ctx->ws_top + 255) & ~(size_t)255) : 0;
+      void* w = avail ? ctx->ws + ((ctx->ws_top + 255) & ~(size_t)255) : nullptr;
+      const size_t need = gemm_packed_c32_bytes(g, ctx->num_sms);
+      if (need > avail) {
+        w = overflow_scratch(ctx, need, s);
+        avail = w ? ctx->ovf_bytes : 0;
+      }
+      const cudaError_t e = tab && w ? launch_gemm_packed_c32(g, w, avail, ctx->num_sms, s, tab) : cudaErrorNotSupported;
+      if (e != cudaErrorNotSupported) {
+        trace_path("  -> packed complex");
+        return cuda_err(e, "packed complex gemm");
+      }
+      cudaGetLastError();
+      ctx->ws_top = top;
+    }
     trace_path("  -> simt");
     // split-K partials (long K, few tiles) go to the free workspace above ws_top
     const size_t off = (ctx->ws_top + 255) & ~(size_t)255;

@@ -607,7 +607,12 @@ struct PackArgs {
   int64_t* c_tab;     // C offset of every row (NULL: no table), from c_str
   int64_t R, K, L, RT, NKT;
   int nr, nk, nl, kfast;
-  int64_t r_ext[MAXG], r_str[MAXG], k_ext[MAXG], k_str[MAXG], l_ext[MAXG], l_str[MAXG], c_str[MAXG];
+  int64_t r_ext[MAXG], r_str[MAXG], k_ext[MAXG], k_str[MAXG], l_ext[MAXG], l_str[MAXG];
+  int nc;             // modes of the C table
+  int64_t c_ext[MAXG], c_str[MAXG];
+  // ComplexF32 through its real 2 x 2 embedding: the modes above are complex
+  // (R and K count real rows and k), rows of A come in pairs (re, -im), (im, re)
+  int a_side;
 };
 
 
@@ -621,7 +626,32 @@ struct PkArgs {
   int S;
 };
 
-template <int NT>
+// One unit of the embedding: 4 consecutive complex k of one row as 8 real
+// values, row kind 0: (re, -im), 1: (im, re), 2: (re, im).
+__device__ __forceinline__ void load_unit_c32(const float2* __restrict__ base, int64_t rowoff, int64_t k0, int64_t K,
+                                              int kfast, int nk, const int64_t* kext, const int64_t* kstr, int kind,
+                                              float (&v)[8]) {
+  float2 c[4];
+  const float2* p = base + rowoff + (rowoff >= 0 && kfast && k0 + 4 <= K ? goff(k0, nk, kext, kstr) : 0);
+  if (rowoff >= 0 && kfast && k0 + 4 <= K && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    c[0] = make_float2(a.x, a.y);
+    c[1] = make_float2(a.z, a.w);
+    c[2] = make_float2(b.x, b.y);
+    c[3] = make_float2(b.z, b.w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      c[i] = rowoff >= 0 && k0 + i < K ? __ldg(base + rowoff + goff(k0 + i, nk, kext, kstr)) : make_float2(0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = kind == 1 ? c[i].y : c[i].x;
+    v[2 * i + 1] = kind == 0 ? -c[i].y : kind == 1 ? c[i].x : c[i].y;
+  }
+}
+
+template <int NT, bool CPLX>
 __device__ __forceinline__ void pack_blob(const PackArgs& p, int64_t b, int warp, int lane) {
   using namespace pk;
   const int64_t kt = b % p.NKT;
@@ -641,8 +671,15 @@ __device__ __forceinline__ void pack_blob(const PackArgs& p, int64_t b, int warp
     if (p.kfast) { row = 8 * vw + (lane & 7); kc = lane >> 3; }
     else { row = 32 * (vw & 3) + lane; kc = vw >> 2; }
     const int64_t r = rt * BM + row;
-    const int64_t roff = r < p.R ? loff + goff(r, p.nr, p.r_ext, p.r_str) : -1;
-    load_unit(p.X, roff, kt * BK + kc * 8, p.K, p.kfast, p.nk, p.k_ext, p.k_str, v[j]);
+    if constexpr (CPLX) {
+      const int64_t rc = p.a_side ? r >> 1 : r;
+      const int64_t roff = r < p.R ? loff + goff(rc, p.nr, p.r_ext, p.r_str) : -1;
+      load_unit_c32(reinterpret_cast<const float2*>(p.X), roff, (kt * BK + kc * 8) >> 1, p.K >> 1, p.kfast, p.nk,
+                    p.k_ext, p.k_str, p.a_side ? (int)(r & 1) : 2, v[j]);
+    } else {
+      const int64_t roff = r < p.R ? loff + goff(r, p.nr, p.r_ext, p.r_str) : -1;
+      load_unit(p.X, roff, kt * BK + kc * 8, p.K, p.kfast, p.nk, p.k_ext, p.k_str, v[j]);
+    }
     so[j] = ((row >> 3) * 4 + kc) * 8 + (row & 7);
   }
 #pragma unroll
@@ -657,7 +694,7 @@ __device__ __forceinline__ void pack_blob(const PackArgs& p, int64_t b, int warp
 // One launch packs A, then B, then fills the C offset tables of the rows of
 // A (M) and B (N) when they are asked for: work unit = one blob or 256
 // table entries, grid-stride over all of them.
-template <int NT>
+template <int NT, bool CPLX>
 __global__ void __launch_bounds__(256) k_pack_split(const __grid_constant__ PackArgs pa,
                                                     const __grid_constant__ PackArgs pb) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -666,14 +703,14 @@ __global__ void __launch_bounds__(256) k_pack_split(const __grid_constant__ Pack
   const int64_t total = na + nb + ta + tb;
   for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
     if (u < na) {
-      pack_blob<NT>(pa, u, warp, lane);
+      pack_blob<NT, CPLX>(pa, u, warp, lane);
     } else if (u < na + nb) {
-      pack_blob<NT>(pb, u - na, warp, lane);
+      pack_blob<NT, CPLX>(pb, u - na, warp, lane);
     } else {
       const bool first = u < na + nb + ta;
       const PackArgs& p = first ? pa : pb;
       const int64_t i = (u - na - nb - (first ? 0 : ta)) * 256 + threadIdx.x;
-      if (i < p.R) p.c_tab[i] = mode_offset(i, p.nr, p.r_ext, p.c_str);
+      if (i < p.R) p.c_tab[i] = mode_offset(i, p.nc, p.c_ext, p.c_str);
     }
   }
 }
@@ -1122,13 +1159,11 @@ static GemmArgs gemm_swapped(const GemmArgs& q) {
   return g;
 }
 
-cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, size_t ws_bytes, int num_sms,
-                               cudaStream_t s, int64_t* ctab) {
+// The packed product of g (its C side, extents in real numbers) whose operands
+// pa and pb describe.
+static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, bool cplx, int nterms, void* workspace,
+                                 size_t ws_bytes, int num_sms, cudaStream_t s, int64_t* ctab) {
   using namespace pk;
-  // consecutive threads store consecutive rows: the rows are the side that has
-  // C's contiguous mode
-  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;
-  if (!gemm_split_supported(g) || (nterms != 2 && nterms != 3)) return cudaErrorNotSupported;
   static std::atomic<unsigned long long> attr2{0}, attr3{0};
   {
     const cudaError_t e = nterms == 2 ? set_smem_once(attr2, k_gemm_packed<2>, Cfg<2>::SMEM_BYTES)
@@ -1162,20 +1197,21 @@ cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, s
   unsigned char* PA = w;
   unsigned char* PB = w + ((bytes_a + 255) & ~(size_t)255);
   float* part = reinterpret_cast<float*>(PB + ((bytes_b + 255) & ~(size_t)255));
-
-  PackArgs pa, pb;
-  pack_args(pa, static_cast<const float*>(g.A), PA, g.M, g.nm, g.m_ext, g.m_sa, g, g.k_sa, g.l_sa);
-  pack_args(pb, static_cast<const float*>(g.B), PB, g.N, g.nn, g.n_ext, g.n_sb, g, g.k_sb, g.l_sb);
+  pa.P = PA;
+  pb.P = PB;
   if (ctab) {
     pa.c_tab = ctab;
     pb.c_tab = ctab + g.M;
-    for (int i = 0; i < g.nm; ++i) pa.c_str[i] = g.m_sc[i];
-    for (int i = 0; i < g.nn; ++i) pb.c_str[i] = g.n_sc[i];
+    pa.nc = g.nm;
+    pb.nc = g.nn;
+    for (int i = 0; i < g.nm; ++i) { pa.c_ext[i] = g.m_ext[i]; pa.c_str[i] = g.m_sc[i]; }
+    for (int i = 0; i < g.nn; ++i) { pb.c_ext[i] = g.n_ext[i]; pb.c_str[i] = g.n_sc[i]; }
   }
   const int64_t units = g.L * (TM + TN) * NKT + (ctab ? (g.M + 255) / 256 + (g.N + 255) / 256 : 0);
   const unsigned gp = (unsigned)std::min<int64_t>(units, (int64_t)num_sms * 8);
-  if (nterms == 2) k_pack_split<2><<<gp, 256, 0, s>>>(pa, pb);
-  else k_pack_split<3><<<gp, 256, 0, s>>>(pa, pb);
+  if (cplx) k_pack_split<3, true><<<gp, 256, 0, s>>>(pa, pb);
+  else if (nterms == 2) k_pack_split<2, false><<<gp, 256, 0, s>>>(pa, pb);
+  else k_pack_split<3, false><<<gp, 256, 0, s>>>(pa, pb);
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -1214,6 +1250,63 @@ cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, s
   k_splitk_tiles<<<(unsigned)std::min<int64_t>(Rt * 64, (int64_t)num_sms * 16), 256, 0, s>>>(t);
   count_launch();
   return cudaGetLastError();
+}
+
+cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, size_t ws_bytes, int num_sms,
+                               cudaStream_t s, int64_t* ctab) {
+  // consecutive threads store consecutive rows: the rows are the side that has
+  // C's contiguous mode
+  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;
+  if (!gemm_split_supported(g) || (nterms != 2 && nterms != 3)) return cudaErrorNotSupported;
+  PackArgs pa, pb;
+  pack_args(pa, static_cast<const float*>(g.A), nullptr, g.M, g.nm, g.m_ext, g.m_sa, g, g.k_sa, g.l_sa);
+  pack_args(pb, static_cast<const float*>(g.B), nullptr, g.N, g.nn, g.n_ext, g.n_sb, g, g.k_sb, g.l_sb);
+  return launch_packed(g, pa, pb, false, nterms, workspace, ws_bytes, num_sms, s, ctab);
+}
+
+// A ComplexF32 product in real numbers: the C side of its 2 x 2 embedding,
+// (2 M) x (2 K) by (2 K) x N, whose result is C's own interleaved storage.
+static bool c32_embedded(GemmArgs& g, const GemmArgs& q) {
+  if (q.nm >= MAXG) return false;
+  g = q;
+  g.M = 2 * q.M;
+  g.K = 2 * q.K;
+  const int at = q.m_sc[0] == 1 ? 0 : 1;   // the part joins a contiguous row mode, or is a mode of its own
+  g.nm = q.nm + at;
+  g.m_ext[0] = 2;
+  g.m_sc[0] = 1;
+  for (int i = 0; i < q.nm; ++i) {
+    g.m_ext[i + at] = i == 0 && at == 0 ? 2 * q.m_ext[0] : q.m_ext[i];
+    g.m_sc[i + at] = i == 0 && at == 0 ? 1 : 2 * q.m_sc[i];
+  }
+  for (int i = 0; i < q.nn; ++i) g.n_sc[i] = 2 * q.n_sc[i];
+  for (int i = 0; i < q.nl; ++i) g.l_sc[i] = 2 * q.l_sc[i];
+  const float one = 1.f;
+  memset(&g.sx, 0, sizeof(g.sx));
+  memcpy(g.sx.b, &one, sizeof(one));
+  return true;
+}
+
+size_t gemm_packed_c32_bytes(const GemmArgs& q, int num_sms) {
+  GemmArgs g = q;
+  g.M = 2 * std::max(q.M, q.N);   // (either side may be the embedded one)
+  g.N = std::min(q.M, q.N);
+  g.K = 2 * q.K;
+  return gemm_packed_bytes(g, 3, num_sms);
+}
+
+cudaError_t launch_gemm_packed_c32(const GemmArgs& q0, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s,
+                                   int64_t* ctab) {
+  const GemmArgs q = q0.n_sc[0] == 1 && q0.m_sc[0] != 1 ? gemm_swapped(q0) : q0;
+  GemmArgs g;
+  if (!q.sx_one || !q.sy_zero || !c32_embedded(g, q) || !gemm_split_supported(g)) return cudaErrorNotSupported;
+  PackArgs pa, pb;
+  pack_args(pa, static_cast<const float*>(q.A), nullptr, g.M, q.nm, q.m_ext, q.m_sa, g, q.k_sa, q.l_sa);
+  pack_args(pb, static_cast<const float*>(q.B), nullptr, g.N, q.nn, q.n_ext, q.n_sb, g, q.k_sb, q.l_sb);
+  pa.a_side = 1;
+  pa.kfast = q.k_sa[0] == 1 && q.k_ext[0] % 4 == 0;
+  pb.kfast = q.k_sb[0] == 1 && q.k_ext[0] % 4 == 0;
+  return launch_packed(g, pa, pb, true, 3, workspace, ws_bytes, num_sms, s, g.nm > 1 || g.nn > 1 ? ctab : nullptr);
 }
 
 // ---------------------------------------------------------------------------

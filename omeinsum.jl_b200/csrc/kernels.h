@@ -98,6 +98,11 @@ cudaError_t launch_c_offsets(GemmArgs& g, int64_t* tab, cudaStream_t s);
 cudaError_t launch_gemm_packed(const GemmArgs& g, int nterms, void* workspace, size_t ws_bytes, int num_sms,
                                cudaStream_t s, int64_t* ctab);
 size_t gemm_packed_bytes(const GemmArgs& g, int nterms, int num_sms);
+// The same for ComplexF32 through its real 2 x 2 embedding (BF16x6 terms); sx = 1
+// and sy = 0 only.  ctab: 2 max(M, N) + min(M, N) entries, or NULL.
+cudaError_t launch_gemm_packed_c32(const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s,
+                                   int64_t* ctab);
+size_t gemm_packed_c32_bytes(const GemmArgs& g, int num_sms);
 // 2-SM tensor-core GEMM fed by TMA tensor maps over the FP32 operands (BF16
 // terms formed in shared memory): single-mode M, N, K and batch groups, each
 // operand contiguous along its row or K mode, 16-byte aligned.  Split-K

@@ -502,7 +502,8 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   // needs more takes its terms from the context's overflow scratch)
   auto packed_gemm_bytes = [&](int j, bool use_sliced) -> size_t {
     const PNode& n = p->nodes[j];
-    if (dtype != OME_F32 || prec == OME_PREC_FP32 || n.args.size() != 2) return 0;
+    const bool c32 = dtype == OME_C32;
+    if ((dtype != OME_F32 && !c32) || prec == OME_PREC_FP32 || n.args.size() != 2) return 0;
     auto labs = [&](int r) -> std::vector<int32_t> {
       std::vector<int32_t> v;
       if (r >= 0) {
@@ -528,7 +529,15 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
         else if (ia && iy) M *= e;
         else if (ib && iy) N *= e;
       }
-    if (M < 256 || N < 256 || K < 512 || 2.0 * M * N * K * L < 1e9) return 0;
+    if (c32) {   // (the real embedding of the longer side)
+      if (M < 128 || N < 128 || K < 128 || 8.0 * M * N * K * L < 1e9) return 0;
+      const double longer = std::max(M, N);
+      N = std::min(M, N);
+      M = 2 * longer;
+      K *= 2;
+    } else if (M < 256 || N < 256 || K < 512 || 2.0 * M * N * K * L < 1e9) {
+      return 0;
+    }
     const double bytes = L * (std::ceil(M / 128) + std::ceil(N / 128)) * std::ceil(K / 32) * 3 * 8192 +
                          74.0 * 256 * 256 * 4 + (M + N) * 8 + 4096;
     return bytes <= (double)((size_t)2 << 30) ? (size_t)bytes : 0;
@@ -811,6 +820,11 @@ int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves&
     if (st.nin == 1) n.x1 = nullptr;
     n.y = at(st.kind[2], st.ref[2]);
     n.yw = wide(st.kind[2], st.ref[2]);
+    // a value that only this program reads is kept in the wider type alone
+    if (which == TINY_FWD && n.yw) {
+      const int up = p->nodes[st.ref[2]].parent;
+      if (up >= 0 && p->nodes[up].tiny && (up != root || count == steps.size())) n.y = nullptr;
+    }
   }
   return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)count, s), "tiny program");
 }

@@ -128,3 +128,28 @@ def test_small_f32_sums_in_double(code, sizes):
     ome.einsum_(c, [to_dev(x, "f32") for x in xs], yd, 2, 3, sizes)
     ome.device_status()
     assert_match(to_np(yd), 2 * want + 3 * y0.astype(np.float64), "f32", 3e-7)
+
+
+@pytest.mark.parametrize("code,sizes", [
+    ("ij,jk->ik", dict(i=128, j=4000, k=257)),           # one row tile, a last column tile of one column
+    ("ji,kj->ki", dict(i=511, j=513, k=513)),            # transposed operands, C contiguous along the second one
+    ("ij,jk->ki", dict(i=1100, j=129, k=900)),
+    ("acbd,cedf->eabf", dict(a=9, b=33, c=13, d=21, e=10, f=51)),   # two modes in every group
+    ("lij,ljk->lik", dict(l=3, i=300, j=260, k=290)),    # a batch mode
+])
+def test_large_c32_on_tensor_cores(code, sizes):
+    """Large ComplexF32 products run on the packed tensor-core kernel through
+    the real embedding: norm-wise below 3e-7 of the ComplexF64 result (BF16x6
+    products summed in FP32 over chunks of 128 real k)."""
+    rng = np.random.default_rng(17)
+    ixs, iy = parse(code)
+    xs = [gen(rng, [sizes[l] for l in ix], "c64") for ix in ixs]
+    want = oracle(ixs, iy, xs, sizes, "c64", wide=True)
+    c = ome.EinCode(ixs, iy)
+    for dev in ([to_dev(x, "c64") for x in xs], [torch.from_numpy(x).cuda() for x in xs]):
+        assert_match(to_np(ome.einsum(c, dev, sizes)), want, "c64", 3e-7)
+        ome.device_status()
+    y0 = gen(rng, [sizes[l] for l in iy], "c64")
+    yd = to_dev(y0, "c64")
+    ome.einsum_(c, [to_dev(x, "c64") for x in xs], yd, 2 + 1j, 3, sizes)   # (general scalars: the CUDA cores)
+    assert_match(to_np(yd), (2 + 1j) * want + 3 * y0.astype(np.complex128), "c64")
