@@ -1,12 +1,14 @@
-// CUDA-core strided batched GEMM over any algebra.
+// Strided batched GEMM over any algebra on the CUDA cores (k_gemm_simt), and in
+// Float64 on the FP64 matrix instructions (k_gemm_dmma).
 //
 // Replaces analyze_binary's permute -> reshape -> (batched) GEMM chain
 // (src/einsum.jl:104-124, src/binaryrules.jl:46-61,94-141, src/utils.jl:162-177,
-// ext/CUDAExt.jl:115-117,156-178) for the element types that have no
-// tensor-core path (Int64, Bool, tropical, FP64, complex) and for the plain
-// FP32 comparison path.  Operands are read in place through per-group mode
-// strides, so no permuted copy is ever materialised; the output permutation
-// is absorbed in the epilogue's strides.
+// ext/CUDAExt.jl:115-117,156-178) for the element types whose arithmetic the
+// tensor cores do not have (Int64, Bool, tropical, FP64, ComplexF64), for
+// ComplexF32 and FP32 products too small for them, and for the plain FP32
+// comparison path.  Operands are read in place through per-group mode strides,
+// so no permuted copy is ever materialised; the output permutation is absorbed
+// in the epilogue's strides.
 #include <cooperative_groups.h>
 #include <string.h>
 #include <algorithm>

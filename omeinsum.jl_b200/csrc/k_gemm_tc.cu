@@ -582,7 +582,8 @@ cudaError_t launch_gemm_split(const GemmArgs& g, int nterms, void* workspace, si
 // the epilogue of one unit overlaps the MMAs of the next.
 // Bound by the tensor pipe.  An MMA of the pair takes 155 clocks with N = 128 and
 // 185 with N = 256 (copies, drains, operand layout and the accumulators' order
-// changed neither), so the tile is the widest there is.
+// changed neither), so the tile is the widest there is: 4096^3 on unaligned rows
+// 822 -> 612 us, 8191^3 6.73 -> 5.09 ms against 128 x 128 tiles of one CTA.
 namespace pk {
 constexpr int BM = 128, BK = 32, CHUNK = 4, XCHUNK = 4 * CHUNK;
 constexpr int TILE_BYTES = BM * BK * 2;     // one term of one operand for one k-step

@@ -496,7 +496,8 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   // children's sizes), split-reduction partials and GEMM workspace; sliced
   // sizes for the forward plan, full sizes for the (unsliced) gradient
   // FP32 binary nodes that the dispatcher sends to the packed-operand
-  // tensor-core GEMM (M, N >= 256, K >= 512, >= 1 GFLOP) need their BF16
+  // tensor-core GEMM (M, N >= 256, K >= 512, >= 1 GFLOP; ComplexF32: M, N, K >=
+  // 128, >= 1 GFLOP, through the real embedding) need their BF16
   // terms in the workspace: L * (M/128 + N/128 tiles) * K/32 k-steps * 24 KB,
   // plus split partials and offset tables (at most 2 GB here; a node that
   // needs more takes its terms from the context's overflow scratch)
