@@ -90,3 +90,34 @@ def test_ring_gradients(n, ext, dt):
     assert_match(to_np(y), v.detach().numpy(), dt, 1e-10 if dt != "f32" else None)
     for g, t in zip(grads, ts):
         assert_match(to_np(g), t.grad.numpy(), dt, 1e-10 if dt != "f32" else None)
+
+
+@pytest.mark.parametrize("dt", ["f32", "c64"])
+@pytest.mark.parametrize("n,ext", [(9, [2, 3]), (17, [2, 3]), (12, [5, 30])])
+def test_float32_trees_in_float64(n, ext, dt):
+    """Trees of eight and more Float32 / ComplexF32 nodes are evaluated in
+    64 bits and rounded once: norm-wise below 1e-7 (half an ulp is 6e-8), also
+    onto old values and for gradients with a cotangent."""
+    rng = np.random.default_rng(500 + n)
+    tree, ixs, sizes = chain(n, ext, rng)
+    wide_t = np.float64 if dt == "f32" else np.complex128
+    xs = [gen(rng, [sizes[l] for l in ix], dt) for ix in ixs]
+    xs = [x / np.sqrt(x.shape[1]).astype(x.real.dtype) for x in xs]
+    ts = [torch.from_numpy(x.astype(wide_t)).requires_grad_() for x in xs]
+    m = torch.eye(sizes[0], dtype=ts[0].dtype)
+    for t in ts:
+        m = m @ t
+    v = torch.diagonal(m)
+    dy = gen(rng, [sizes[0]], dt)
+    v.backward(torch.from_numpy(dy.astype(wide_t)))
+    want = v.detach().numpy()
+    dev = [to_dev(x, dt) for x in xs]
+    assert_match(to_np(tree(*dev)), want, dt, 1e-7)
+    y0 = gen(rng, [sizes[0]], dt)
+    y = to_dev(y0, dt)
+    ome.einsum_(tree, dev, y, 2, 3)
+    assert_match(to_np(y), 2 * want + 3 * y0.astype(wide_t), dt, 3e-7)
+    got, grads = ome.cost_and_gradient(tree, dev, dy=to_dev(dy, dt))
+    assert_match(to_np(got), want, dt, 1e-7)
+    for g, t in zip(grads, ts):
+        assert_match(to_np(g), t.grad.numpy(), dt, 1e-7)
