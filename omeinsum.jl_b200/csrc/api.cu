@@ -498,6 +498,16 @@ static int gemm_kernel_choice(const GemmArgs& g) {
   return g.M >= 256 && g.N >= 256 && g.K >= 512 && flops >= 1e9 ? 1 : 0;
 }
 
+// Float32 nodes of sliced trees (ome_ctx::fixed_sums).  A network's value is a
+// sum with cancellations: over 64 sets of inputs of a sliced 160-vertex network
+// the roundings of its nodes end up as 2e-7 .. 3.5e-5 of the value, and two
+// equally exact ways of summing its nodes as up to 7.7e-5 between them.  Such a
+// tree's nodes therefore keep one order of summation whatever kernel or tile
+// serves them best: products on the tensor cores are summed over 8 stages, main
+// and cross terms joined (k_gemm_packed, k_gemm_bf16x3), K is cut by the count
+// of 128 x 128 tiles, operands are not exchanged where that would move a cut,
+// and small nodes are summed in Float32 term by term (k_loop_thread, k_tiny).
+
 // Scratch of `need` bytes for a packed GEMM whose operands do not fit the
 // workspace: the context's overflow buffer, grown (64 MiB granules) when it
 // is smaller, but never during stream capture and never past a quarter of
@@ -602,6 +612,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
     g.sy = sy;
     g.sy_zero = sy_zero;
     g.sx_one = scalar_is_one(dt, sx);
+    g.fixed_sums = ctx->fixed_sums && dt == OME_F32;
     trace_path("gemm M=%lld N=%lld K=%lld L=%lld modes=%d/%d/%d/%d afast=%d bfast=%d prec=%d", (long long)M,
                (long long)N, (long long)K, (long long)L, gm.n, gn.n, gk.n, gl.n, g.a_m_fast, g.b_n_fast, prec);
     // batches of small GEMMs with the batch mode innermost in every tensor
@@ -642,7 +653,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       const double macs = (double)M * (double)N * (double)K * (double)L;
       const bool k_scattered =
           g.nk > 1 && (g.k_ext[0] % 8 != 0 || g.k_sa[0] != 1 || g.k_sb[0] != 1);
-      if (choice == 0 && macs <= (k_scattered ? 0x1p28 : 0x1p25)) {
+      if (choice == 0 && !g.fixed_sums && macs <= (k_scattered ? 0x1p28 : 0x1p25)) {
         trace_path("  -> small");
         cudaError_t e = launch_gemm_small_f32(g, w, avail, ctx->num_sms, s);
         if (e != cudaErrorNotSupported) return cuda_err(e, "small gemm");
@@ -662,7 +673,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       // operands (its products run 1.3 times faster than beside converters):
       // 4096^3 675 -> 600 us, 3072^3 281 -> 269; 2304^3 130 against 138,
       // 8192 x 512 x 8192 358 against 431
-      const bool prefer_packed = choice == 2 && K >= 2048 && M * N >= 1536 * (M + N) &&
+      const bool prefer_packed = choice == 2 && !g.fixed_sums && K >= 2048 && M * N >= 1536 * (M + N) &&
                                  gemm_packed_bytes(g, nterms, ctx->num_sms) <= avail;
       if (choice == 1 || prefer_packed) {
         cudaError_t e = packed();

@@ -327,6 +327,9 @@ struct GemmArgs {
   // evaluating a mixed-radix offset per element
   const int64_t* m_tab_c;
   const int64_t* n_tab_c;
+  // Float32 node of a sliced tree: every sum in the order that does not depend
+  // on the kernel's tiles (see run_binary)
+  int fixed_sums;
 };
 
 // Offset of flat index i over modes (column-major, first mode fastest).

@@ -15,6 +15,7 @@ struct ome_ctx {
   size_t ws_top;     // bump pointer; reset by every top-level call
   char* ovf;         // operand scratch of packed GEMMs that do not fit the workspace
   size_t ovf_bytes;  // (grown on demand outside stream capture; freed with the context)
+  bool fixed_sums;   // the nodes of a sliced Float32 tree are being evaluated (see run_binary)
 };
 
 namespace ome {

@@ -570,10 +570,14 @@ cudaError_t launch_gemm_split(const GemmArgs& g, int nterms, void* workspace, si
 //    lane), in the peer it tells the leader that a stage has landed;
 //  * TMEM holds one main (t0*t0) and one cross-term accumulator of 256 columns.
 //    A stage's cross products go first: while they run, warps 0-7 of both CTAs
-//    drain the main accumulator of the chunk before (CHUNK stages) into FP32
+//    drain the main accumulator of the chunk before (4 stages) into FP32
 //    running sums in registers (thread = one row x 128 columns) with
 //    round-to-nearest adds.  The cross terms are 2^-8 of the main ones and so is
-//    the round-off of their accumulation: they are drained every fourth chunk;
+//    the round-off of their accumulation: they are drained every fourth chunk.
+//    For the nodes of a sliced tree (GemmArgs::fixed_sums) both are drained
+//    together after 8 stages and joined before the add, as k_gemm_bf16x3 does:
+//    the same time (16384 x 4096 x 4096 and the rest of a sliced 160-vertex
+//    network 15.2 ms either way), error at K = 4097 2.4e-7 instead of 1.7e-7;
 //  * the same warps store the tile (αβ epilogue, or a split partial).
 // The kernel is persistent over work units: the first F tiles (whole waves of
 // the clusters) are computed whole, the remaining tiles are cut into S K-splits
@@ -585,7 +589,7 @@ cudaError_t launch_gemm_split(const GemmArgs& g, int nterms, void* workspace, si
 // changed neither), so the tile is the widest there is: 4096^3 on unaligned rows
 // 822 -> 612 us, 8191^3 6.73 -> 5.09 ms against 128 x 128 tiles of one CTA.
 namespace pk {
-constexpr int BM = 128, BK = 32, CHUNK = 4, XCHUNK = 4 * CHUNK;
+constexpr int BM = 128, BK = 32;
 constexpr int TILE_BYTES = BM * BK * 2;     // one term of one operand for one k-step
 constexpr int NDRAIN = 256;                 // drain / epilogue warps 0-7
 constexpr int NTHREADS = NDRAIN + 64;       // + producer warp 8 + MMA warp 9
@@ -625,6 +629,8 @@ struct PkArgs {
   int64_t RA, RB;              // 128-row tiles of A and B
   int64_t TM, TN, NKT, tiles, F, ksplit, units;
   int S;
+  int chunk, xchunk;           // stages between two drains of the main and of the cross accumulator (powers of two)
+  int swapped;                 // A and B are the caller's B and A: cross products in the caller's order
 };
 
 // One unit of the embedding: 4 consecutive complex k of one row as 8 real
@@ -937,14 +943,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
         decode(u, l, mt, nt, kb, ke, slot);
         const int nk = (int)(ke - kb);
         for (int j = 0; j < nk; ++j, ++it) {
-          const bool first = j % CHUNK == 0, xfirst = j % XCHUNK == 0;
+          const bool first = (j & (t.chunk - 1)) == 0, xfirst = (j & (t.xchunk - 1)) == 0;
           const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
           bool in = true;
           if (xfirst && xc >= 1) in = mbar_wait_cl(xdrained, (xc - 1) & 1, abort_flag);
           in = in && mbar_wait(&full[s], par, abort_flag) && mbar_wait_cl(&peer_full[s], par, abort_flag);
           if (!__all_sync(0xffffffffu, in)) { ok = false; break; }
           tc_fence_after();
-          const bool last = j % CHUNK == CHUNK - 1 || j == nk - 1;
+          const bool last = (~j & (t.chunk - 1)) == 0 || j == nk - 1;
           const uint32_t sa = sbase + s * STAGE_BYTES, sb = sa + BLOB;
           if (elect_one()) {
 #pragma unroll
@@ -954,8 +960,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
               for (int d = 1; d < NT; ++d)
 #pragma unroll
                 for (int i = 0; i <= d; ++i) {
-                  umma_bf16_pair(tmem_cross, umma_desc(sa + i * TILE_BYTES + kk * 256),
-                                 umma_desc(sb + (d - i) * TILE_BYTES + kk * 256), start ? 0u : 1u, IDESC);
+                  const int ia = t.swapped ? d - i : i;
+                  umma_bf16_pair(tmem_cross, umma_desc(sa + ia * TILE_BYTES + kk * 256),
+                                 umma_desc(sb + (d - ia) * TILE_BYTES + kk * 256), start ? 0u : 1u, IDESC);
                   start = false;
                 }
             }
@@ -976,7 +983,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
           }
           __syncwarp();
           if (last) ++gc;
-          if (j % XCHUNK == XCHUNK - 1 || j == nk - 1) ++xc;
+          if ((~j & (t.xchunk - 1)) == 0 || j == nk - 1) ++xc;
         }
       }
       // every MMA this warp issued must finish before TMEM is freed, and the
@@ -1003,7 +1010,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
     for (int64_t u = cid; u < t.units; u += ncl) {
       int64_t l, mt, nt, kb, ke, slot;
       decode(u, l, mt, nt, kb, ke, slot);
-      const int nch = (int)((ke - kb + CHUNK - 1) / CHUNK);
+      const int nch = (int)((ke - kb + t.chunk - 1) / t.chunk);
       it += (uint32_t)(ke - kb);
       float sum[128];
 #pragma unroll
@@ -1022,11 +1029,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(done);
       };
+      auto drain_pair = [&]() {   // both, joined before they are added
+#pragma unroll
+        for (int hh = 0; hh < 8; ++hh) {
+          uint32_t rm[16], rc[16];
+          __syncwarp();
+          tmem_ld16(tmem_main + lane_off + (uint32_t)(col0 + 16 * hh), rm);
+          tmem_ld16(tmem_cross + lane_off + (uint32_t)(col0 + 16 * hh), rc);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sum[16 * hh + j] += __uint_as_float(rm[j]) + __uint_as_float(rc[j]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_remote(lead_drained);
+          mbar_arrive_remote(lead_xdrained);
+        }
+      };
       for (int ci = 0; ci < nch; ++ci, ++gc) {
         if (!__all_sync(0xffffffffu, mbar_wait_cl(chunk_done, gc & 1, abort_flag))) { ok = false; break; }
         tc_fence_after();
-        drain(tmem_main, lead_drained);
-        if (ci % (XCHUNK / CHUNK) == XCHUNK / CHUNK - 1 || ci == nch - 1) drain(tmem_cross, lead_xdrained);
+        if (t.xchunk == t.chunk) {
+          drain_pair();
+        } else {
+          drain(tmem_main, lead_drained);
+          if ((~ci & (t.xchunk / t.chunk - 1)) == 0 || ci == nch - 1) drain(tmem_cross, lead_xdrained);
+        }
       }
       if (!ok) break;
       if (slot >= 0) {
@@ -1162,8 +1190,8 @@ static GemmArgs gemm_swapped(const GemmArgs& q) {
 
 // The packed product of g (its C side, extents in real numbers) whose operands
 // pa and pb describe.
-static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, bool cplx, int nterms, void* workspace,
-                                 size_t ws_bytes, int num_sms, cudaStream_t s, int64_t* ctab) {
+static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, bool cplx, bool swapped, int nterms,
+                                 void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s, int64_t* ctab) {
   using namespace pk;
   static std::atomic<unsigned long long> attr2{0}, attr3{0};
   {
@@ -1185,6 +1213,15 @@ static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, 
   if (Rt > 0) {
     S = std::max<int64_t>(1, G / Rt);
     S = std::min<int64_t>(S, std::max<int64_t>(1, NKT / 8));
+  }
+  if (g.fixed_sums) {
+    // K is cut where 128 x 128 tiles on all SMs would be (only if there are
+    // fewer of them than SMs)
+    const int64_t t128 = g.L * TM * TN;
+    S = t128 < num_sms ? std::min<int64_t>(num_sms / t128, std::max<int64_t>(1, NKT / 8)) : 1;
+    if (tiles * S > G) S = 1;
+    F = 0;
+    Rt = tiles;
   }
   const int64_t ksplit = (NKT + S - 1) / S;
   S = (NKT + ksplit - 1) / ksplit;
@@ -1236,6 +1273,9 @@ static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, 
   t.F = F;
   t.S = (int)S;
   t.ksplit = ksplit;
+  t.swapped = swapped;
+  t.chunk = g.fixed_sums ? 8 : 4;
+  t.xchunk = g.fixed_sums ? 8 : 16;
   t.units = F + Rt * S;
   const unsigned grid = (unsigned)(2 * std::min<int64_t>(t.units, G));
   // plain launches: a GEMM block started early would hold its SM's shared
@@ -1257,12 +1297,13 @@ cudaError_t launch_gemm_packed(const GemmArgs& q, int nterms, void* workspace, s
                                cudaStream_t s, int64_t* ctab) {
   // consecutive threads store consecutive rows: the rows are the side that has
   // C's contiguous mode
-  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;
+  const bool swapped = q.n_sc[0] == 1 && q.m_sc[0] != 1;
+  const GemmArgs g = swapped ? gemm_swapped(q) : q;
   if (!gemm_split_supported(g) || (nterms != 2 && nterms != 3)) return cudaErrorNotSupported;
   PackArgs pa, pb;
   pack_args(pa, static_cast<const float*>(g.A), nullptr, g.M, g.nm, g.m_ext, g.m_sa, g, g.k_sa, g.l_sa);
   pack_args(pb, static_cast<const float*>(g.B), nullptr, g.N, g.nn, g.n_ext, g.n_sb, g, g.k_sb, g.l_sb);
-  return launch_packed(g, pa, pb, false, nterms, workspace, ws_bytes, num_sms, s, ctab);
+  return launch_packed(g, pa, pb, false, swapped, nterms, workspace, ws_bytes, num_sms, s, ctab);
 }
 
 // A ComplexF32 product in real numbers: the C side of its 2 x 2 embedding,
@@ -1307,7 +1348,7 @@ cudaError_t launch_gemm_packed_c32(const GemmArgs& q0, void* workspace, size_t w
   pa.a_side = 1;
   pa.kfast = q.k_sa[0] == 1 && q.k_ext[0] % 4 == 0;
   pb.kfast = q.k_sb[0] == 1 && q.k_ext[0] % 4 == 0;
-  return launch_packed(g, pa, pb, true, 3, workspace, ws_bytes, num_sms, s, g.nm > 1 || g.nn > 1 ? ctab : nullptr);
+  return launch_packed(g, pa, pb, true, false, 3, workspace, ws_bytes, num_sms, s, g.nm > 1 || g.nn > 1 ? ctab : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1950,7 +1991,7 @@ size_t gemm_tma2_bytes(const GemmArgs& g, int num_sms) {
 
 cudaError_t launch_gemm_tma2(const GemmArgs& q, int nterms, void* workspace, size_t ws_bytes, int num_sms,
                              cudaStream_t s) {
-  const GemmArgs g = q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;   // (as in launch_gemm_packed)
+  const GemmArgs g = !q.fixed_sums && q.n_sc[0] == 1 && q.m_sc[0] != 1 ? gemm_swapped(q) : q;   // (as in launch_gemm_packed)
   if ((nterms != 2 && nterms != 3) || !gemm_tma2_applies(g)) return cudaErrorNotSupported;
   const bool ak = g.k_sa[0] == 1, bk = g.k_sb[0] == 1;
   alignas(64) CUtensorMap ma, mb;

@@ -145,8 +145,10 @@ size_t tiny_wide_size(ome_dtype dt);
 // if it does not fit a TinyNode.
 struct HView;
 bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y);
-// Runs nodes[0..n) (level[i] ascending); one launch per 100 nodes.
-cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, cudaStream_t s);
+// Runs nodes[0..n) (level[i] ascending); one launch per 100 nodes.  plain: sums
+// and results in the element type itself, with k_loop_thread's arithmetic (for
+// nodes without TINY_WARP; Float32).
+cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, bool plain, cudaStream_t s);
 
 // Read and clear the CUDA-core GEMM's split-partial self-check flag.
 int simt_bounds_flag();

@@ -81,6 +81,7 @@ struct ome_plan {
   size_t fwd_bytes = 0, grad_bytes = 0;     // plus per-node dispatch scratch
   size_t esize = 0;
   size_t wsize = 0;                // bytes of the wider type; 0 if it is the element type
+  bool fixed_sums = false;         // sliced Float32: every node's sums as a call of its own computes them
   // steps of the tiny programs, levels ascending: forward on sliced and on
   // full sizes, reverse sweep; programs built for the last input strides seen
   // (several threads may evaluate one plan)
@@ -245,6 +246,16 @@ bool tiny_step(const ome_plan* p, const std::vector<std::vector<int32_t>>& xs, c
       if (xs.size() == 2 && !contains(y, l) && !contains(xs[1 - i], l) && p->ext.at(l) != 1) return false;
       visit(l);
     }
+  if (p->fixed_sums) {   // only what k_loop_thread evaluates
+    double terms = 1, m = 1, n = 1;
+    for (int32_t l : seen) {
+      const double e = (double)p->ext.at(l);
+      if (!contains(y, l)) terms *= e;
+      else if (!contains(xs.back(), l)) m *= e;
+      else if (!contains(xs[0], l)) n *= e;
+    }
+    if (terms > 16 || (xs.size() == 2 && m >= 16 && n >= 16 && terms >= 8)) return false;
+  }
   return work >= 1 && work <= (double)TINY_WORK;
 }
 
@@ -380,7 +391,8 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   p->dt = dtype;
   p->prec = prec;
   p->esize = dtype_size(dtype);
-  p->wsize = tiny_wide_size(dtype) == p->esize ? 0 : tiny_wide_size(dtype);
+  p->fixed_sums = dtype == OME_F32 && nsliced > 0;
+  p->wsize = p->fixed_sums || tiny_wide_size(dtype) == p->esize ? 0 : tiny_wide_size(dtype);
   p->ninputs = ninputs;
   for (int i = 0; i < nlabels; ++i) {
     if (label_extents[i] < 0) {
@@ -827,7 +839,7 @@ int run_tiny(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leaves&
       if (up >= 0 && p->nodes[up].tiny && (up != root || count == steps.size())) n.y = nullptr;
     }
   }
-  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)count, s), "tiny program");
+  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)count, p->fixed_sums, s), "tiny program");
 }
 
 // The forward values of every node but the root: the tiny program, then the
@@ -868,6 +880,11 @@ int run_forward(ome_ctx* ctx, ome_plan* p, cudaStream_t s, int which, const Leav
 int run_slices(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& inputs, int64_t b, int64_t e,
                char* acc, const Scalar& sx) {
   const ome_dtype dt = p->dt;
+  struct Fixed {   // (see run_binary)
+    ome_ctx* c;
+    Fixed(ome_ctx* ctx, bool on) : c(ctx) { c->fixed_sums = on; }
+    ~Fixed() { c->fixed_sums = false; }
+  } fixed(ctx, p->fixed_sums);
   const Scalar one = scalar_one(dt), zero = scalar_zero(dt);
   const int root = (int)p->nodes.size() - 1;
   const PNode& rn = p->nodes[root];
@@ -934,7 +951,7 @@ int widen_inputs(ome_ctx* ctx, ome_plan* p, cudaStream_t s, const Leaves& in, st
     nodes[t].x0 = in.data[t];
     nodes[t].yw = ctx->ws + p->wide_in[t];
   }
-  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)nodes.size(), s), "inputs to Float64");
+  return cuda_err(launch_tiny(p->dt, nodes.data(), prog->level.data(), (int)nodes.size(), false, s), "inputs to Float64");
 }
 
 }  // namespace
@@ -1126,7 +1143,7 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
         nodes[t].flags |= TINY_WIDE0;
         nodes[t].y = dxs[t];
       }
-      rc = cuda_err(launch_tiny(dt, nodes.data(), prog->level.data(), (int)nodes.size(), s), "gradients from Float64");
+      rc = cuda_err(launch_tiny(dt, nodes.data(), prog->level.data(), (int)nodes.size(), false, s), "gradients from Float64");
       if (rc) return rc;
       return cuda_err(launch_acc64_store(dt, y, ctx->ws + p->wide_y, rn.numel, one, zero, 1, s), "output from Float64");
     }

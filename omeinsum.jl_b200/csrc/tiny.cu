@@ -82,10 +82,9 @@ __device__ __forceinline__ int32_t tiny_digit(uint32_t& r, uint32_t ext) {
   return d;
 }
 
-template <class A, int CAP>
+template <class A, class WA, int CAP>
 __global__ void __launch_bounds__(TINY_THREADS, 1) k_tiny(const __grid_constant__ TinyArgs<CAP> a) {
   using T = typename A::T;
-  using WA = typename TinyWide<A>::W;
   using W = typename WA::T;
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   const int lane = threadIdx.x & 31;
@@ -154,8 +153,12 @@ __global__ void __launch_bounds__(TINY_THREADS, 1) k_tiny(const __grid_constant_
           for (int u = 0; u < U; ++u)
             if (jb + u * step < n.n_in) {
               W p = tiny_conj(tiny_as<W>(v0[u]), c0);
-              if (two) p = WA::mul(p, tiny_conj(tiny_as<W>(v1[u]), c1));
-              acc = WA::add(acc, p);
+              if constexpr (std::is_same<WA, AlgF32>::value) {   // (as k_loop_thread adds a product)
+                acc = two ? WA::fma(p, v1[u], acc) : WA::add(acc, p);
+              } else {
+                if (two) p = WA::mul(p, tiny_conj(tiny_as<W>(v1[u]), c1));
+                acc = WA::add(acc, p);
+              }
             }
         }
       };
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(TINY_THREADS, 1) k_tiny(const __grid_constant_
   }
 }
 
-template <class A, int CAP>
+template <class A, class WA, int CAP>
 cudaError_t launch_tiny_t(const TinyNode* nodes, const int* level, int n, cudaStream_t s) {
   TinyArgs<CAP> a;
   a.nlevels = 0;
@@ -214,11 +217,11 @@ cudaError_t launch_tiny_t(const TinyNode* nodes, const int* level, int n, cudaSt
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(attr.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(k_tiny<A, CAP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(k_tiny<A, WA, CAP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     attr.fetch_or(bit, std::memory_order_release);
   }
-  e = cudaLaunchKernelEx(&cfg, k_tiny<A, CAP>, a);
+  e = cudaLaunchKernelEx(&cfg, k_tiny<A, WA, CAP>, a);
   count_launch();
   return e;
 }
@@ -290,7 +293,7 @@ bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y) {
   return put(outer, 0) && put(inner, outer.n);
 }
 
-cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, cudaStream_t s) {
+cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, int n, bool plain, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   for (int b = 0; b < n && e == cudaSuccess;) {
     // at most TINY_CAP nodes and TINY_LEVELS levels a launch
@@ -304,10 +307,13 @@ cudaError_t launch_tiny(ome_dtype dt, const TinyNode* nodes, const int* level, i
     }
     KernelTimer kt(s, "k_tiny");
     e = cudaErrorInvalidValue;
-    if (c <= TINY_CAP_SMALL) {
-      OME_DISPATCH(dt, ALG, e = (launch_tiny_t<ALG, TINY_CAP_SMALL>(nodes + b, level + b, c, s)));
+    if (plain && dt == OME_F32) {
+      e = c <= TINY_CAP_SMALL ? launch_tiny_t<AlgF32, AlgF32, TINY_CAP_SMALL>(nodes + b, level + b, c, s)
+                              : launch_tiny_t<AlgF32, AlgF32, TINY_CAP>(nodes + b, level + b, c, s);
+    } else if (c <= TINY_CAP_SMALL) {
+      OME_DISPATCH(dt, ALG, e = (launch_tiny_t<ALG, TinyWide<ALG>::W, TINY_CAP_SMALL>(nodes + b, level + b, c, s)));
     } else {
-      OME_DISPATCH(dt, ALG, e = (launch_tiny_t<ALG, TINY_CAP>(nodes + b, level + b, c, s)));
+      OME_DISPATCH(dt, ALG, e = (launch_tiny_t<ALG, TinyWide<ALG>::W, TINY_CAP>(nodes + b, level + b, c, s)));
     }
     b += c;
   }
