@@ -604,13 +604,18 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   p->dy_off = g;
   p->grad_arena = g + ((size_t)p->nodes[root].numel * p->esize + 511);
   p->grad_bytes = ((p->grad_arena + 255) & ~(size_t)255) + scratch_grad;
-  // Small trees in Float64: every value is then rounded to 32 bits once, at the
-  // end, where the roundings of a hundred nodes are amplified by the network's
-  // cancellations (a 100-vertex network's gradients 7e-7 off), and at this size
-  // (2^26 multiply-adds are 8 us of the FP64 pipe) the launches set the time
-  // (below eight nodes the two conversions' launches would be felt).
+  // Trees of up to 2^32 multiply-adds in Float64: every value is then rounded to
+  // 32 bits once, at the end, where the roundings of a hundred nodes are
+  // amplified by the network's cancellations.  Over 12 sets of inputs each of 26
+  // networks between 2^26 and 2^32, with and without gradients, Float32 nodes
+  // leave 1e-7 .. 4e-5 and which of two evaluations is the nearer one is chance;
+  // Float64 leaves 1e-8 .. 5e-8.  Up to 2^26 (8 us of the FP64 pipe) the launches
+  // set the time; 2^29.8 value and gradients 1.00 -> 1.19 ms, 2^31.1 1.15 -> 1.67
+  // and its value alone 0.22 -> 0.41; above, Float64 would be most of the time.
+  // Below eight nodes the two conversions' launches would be felt.  The second
+  // plan's buffers may take 1 GiB.
   if ((dtype == OME_F32 || dtype == OME_C32) && prec != OME_PREC_FP32 && !sliced && nnodes >= 8 &&
-      plan_work(p) <= 0x1p26) {
+      plan_work(p) <= 0x1p32) {
     bool small = true;
     for (auto& l : p->in_labels) {
       double n = 1;
@@ -620,7 +625,12 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
     ome_plan* w = nullptr;
     const ome_dtype wt = dtype == OME_F32 ? OME_F64 : OME_C64;
     if (small && ome_plan_create(ctx, wt, ninputs, input_nlabels, input_labels, nnodes, node_nargs, node_args, node_niy,
-                                 node_iy, nlabels, label_ids, label_extents, 0, nullptr, prec, &w) == OME_OK) {
+                                 node_iy, nlabels, label_ids, label_extents, 0, nullptr, prec, &w) == OME_OK &&
+        w->grad_bytes > (size_t)1 << 30) {
+      delete w;
+      w = nullptr;
+    }
+    if (w) {
       p->wide.reset(w);
       size_t at = 0;
       auto take = [&](int64_t n) {
