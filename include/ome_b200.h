@@ -188,8 +188,14 @@ OME_API int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs,
                     ome_plan** out);
 OME_API int ome_plan_destroy(ome_plan* plan);
 
-/* Peak workspace bytes the plan needs (forward only / forward+gradient). */
+/* Peak workspace bytes of the plan (forward only / forward+gradient). */
 OME_API int ome_plan_peak_bytes(const ome_plan* plan, size_t* forward_bytes, size_t* grad_bytes);
+
+/* The least workspace that it runs in.  Less than the peak for OME_F32 and
+ * OME_C32 trees that are evaluated in 64 bits and rounded once (unsliced, eight
+ * nodes or more, at most 2^32 multiply-adds, not OME_PREC_FP32): below the peak
+ * their nodes are evaluated one by one in their own type. */
+OME_API int ome_plan_min_bytes(const ome_plan* plan, size_t* forward_bytes, size_t* grad_bytes);
 
 /* Evaluate the tree: y <- sy*y + sx*tree(inputs).  inputs[t] are column-major
  * contiguous device buffers; y is column-major contiguous.  With slices, the
@@ -337,8 +343,8 @@ OME_API int ome_graph_destroy(ome_graph* graph);
  * slot is free and the plan's peak workspace bytes (ome_plan_peak_bytes:
  * forward, or forward+gradient for gradient jobs) fit a slot's share; a job
  * above a share but within the budget waits until every slot is idle and runs
- * alone in a workspace of its own size; jobs above the budget
- * (OME_JOB_REJECTED_MEMORY) or with more than max_job_work multiply-adds
+ * alone in a workspace of its own size; jobs whose least workspace
+ * (ome_plan_min_bytes) is above the budget (OME_JOB_REJECTED_MEMORY) or with more than max_job_work multiply-adds
  * (OME_JOB_REJECTED_WORK; max_job_work <= 0: no cap) are rejected at
  * admission.  Admission and retirement happen in ome_server_poll, which never
  * blocks on the device. */

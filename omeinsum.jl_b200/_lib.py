@@ -28,6 +28,7 @@ EXPORTS = [
     "ome_batch_info", "ome_batch_destroy", "ome_batch_graph_create", "ome_graph_launch", "ome_graph_destroy",
     "ome_server_create", "ome_server_submit", "ome_server_poll", "ome_server_stats", "ome_server_clock", "ome_server_destroy",
     "ome_treesa", "ome_greedy", "ome_slice_greedy", "ome_plan_execute_strided", "ome_plan_gradient_strided",
+    "ome_plan_min_bytes",
 ]
 
 JOB_COMPLETED, JOB_FAILED, JOB_REJECTED_MEMORY, JOB_REJECTED_WORK = range(4)
@@ -107,6 +108,7 @@ def load() -> C.CDLL:
                                         C.c_int32, i32p, i64p, C.c_int32, i32p, C.c_int32, C.POINTER(P)]
         lib.ome_plan_destroy.argtypes = [P]
         lib.ome_plan_peak_bytes.argtypes = [P, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
+        lib.ome_plan_min_bytes.argtypes = [P, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
         lib.ome_plan_execute.argtypes = [P, P, P, C.POINTER(P), P, P, P]
         lib.ome_plan_gradient.argtypes = [P, P, P, C.POINTER(P), P, P, C.POINTER(P)]
         lib.ome_plan_execute_strided.argtypes = [P, P, P, C.POINTER(P), i64p, P, P, P]

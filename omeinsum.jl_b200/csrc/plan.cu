@@ -78,7 +78,8 @@ struct ome_plan {
   size_t acc_off = 0, tmp_off = 0;  // FP64 accumulator and root temporary (sliced)
   size_t dy_off = 0;                        // root cotangent buffer (gradient)
   size_t arena_bytes = 0, grad_arena = 0;  // planned buffers (forward / gradient)
-  size_t fwd_bytes = 0, grad_bytes = 0;     // plus per-node dispatch scratch
+  size_t fwd_bytes = 0, grad_bytes = 0;     // plus per-node dispatch scratch: the least it runs in
+  size_t fwd_peak = 0, grad_peak = 0;       // with the buffers of the evaluation in Float64 (`wide`)
   size_t esize = 0;
   size_t wsize = 0;                // bytes of the wider type; 0 if it is the element type
   bool fixed_sums = false;         // sliced Float32: every node's sums as a call of its own computes them
@@ -604,6 +605,8 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
   p->dy_off = g;
   p->grad_arena = g + ((size_t)p->nodes[root].numel * p->esize + 511);
   p->grad_bytes = ((p->grad_arena + 255) & ~(size_t)255) + scratch_grad;
+  p->fwd_peak = p->fwd_bytes;
+  p->grad_peak = p->grad_bytes;
   // Trees of up to 2^32 multiply-adds in Float64: every value is then rounded to
   // 32 bits once, at the end, where the roundings of a hundred nodes are
   // amplified by the network's cancellations.  Over 12 sets of inputs each of 26
@@ -647,8 +650,8 @@ int ome_plan_create(ome_ctx* ctx, ome_dtype dtype, int32_t ninputs, const int32_
       p->wide_y = take(p->nodes[root].numel);
       p->wide_dy = take(p->nodes[root].numel);
       p->wide_base = at;
-      p->fwd_bytes = std::max(p->fwd_bytes, at + w->fwd_bytes);
-      p->grad_bytes = std::max(p->grad_bytes, at + w->grad_bytes);
+      p->fwd_peak = std::max(p->fwd_bytes, at + w->fwd_bytes);
+      p->grad_peak = std::max(p->grad_bytes, at + w->grad_bytes);
       for (int which : {TINY_WIDEN, TINY_NARROW})
         for (int t = 0; t < ninputs; ++t) {
           TinyStep st;
@@ -670,6 +673,13 @@ int ome_plan_destroy(ome_plan* plan) {
 }
 
 int ome_plan_peak_bytes(const ome_plan* plan, size_t* forward_bytes, size_t* grad_bytes) {
+  if (!plan) return set_err(OME_INVALID_ARGUMENT, "plan is NULL");
+  if (forward_bytes) *forward_bytes = plan->fwd_peak;
+  if (grad_bytes) *grad_bytes = plan->grad_peak;
+  return OME_OK;
+}
+
+int ome_plan_min_bytes(const ome_plan* plan, size_t* forward_bytes, size_t* grad_bytes) {
   if (!plan) return set_err(OME_INVALID_ARGUMENT, "plan is NULL");
   if (forward_bytes) *forward_bytes = plan->fwd_bytes;
   if (grad_bytes) *grad_bytes = plan->grad_bytes;
@@ -982,7 +992,7 @@ int ome_plan_execute_strided(ome_ctx* ctx, ome_plan* p, void* stream, const void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const ome_dtype dt = p->dt;
   const Scalar sx = scalar_from(dt, sxp), sy = scalar_from(dt, syp);
-  if (p->wide) {
+  if (p->wide && ctx->ws_bytes >= p->fwd_peak) {
     std::vector<const void*> win;
     bool done;
     int rc = widen_inputs(ctx, p, s, inputs, win, &done);
@@ -1128,7 +1138,7 @@ int ome_plan_gradient_strided(ome_ctx* ctx, ome_plan* p, void* stream, const voi
   const Scalar one = scalar_one(dt), zero = scalar_zero(dt);
   const int root = (int)p->nodes.size() - 1;
   const PNode& rn = p->nodes[root];
-  if (p->wide) {
+  if (p->wide && ctx->ws_bytes >= p->grad_peak) {
     std::vector<const void*> win;
     bool done;
     int rc = widen_inputs(ctx, p, s, inputs, win, &done);

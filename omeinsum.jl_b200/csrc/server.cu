@@ -11,8 +11,9 @@
 // slot is free and the plan's peak workspace bytes (ome_plan_peak_bytes) fit a
 // share; a job above a share but within the whole budget waits until every
 // slot is idle and then runs alone in a workspace of its own size (the slots'
-// workspaces are released first); jobs above the budget, or above the optional
-// work cap, are rejected at admission.  A slot's thread issues the job's
+// workspaces are released first); jobs whose least workspace
+// (ome_plan_min_bytes) is above the budget, or above the optional work cap, are
+// rejected at admission.  A slot's thread issues the job's
 // kernels (ome_plan_execute, or ome_plan_gradient for gradient jobs, which run
 // unsliced as src/bp.jl:26-28 does) so that a large job's host-side issue never
 // blocks admission; completion is the job's event on the slot's stream,
@@ -229,7 +230,11 @@ void admit(ome_server* s) {
     }
     size_t fwd = 0, grad = 0;
     ome_plan_peak_bytes(j->plan, &fwd, &grad);
-    const size_t need = j->dxs.empty() ? fwd : grad;
+    size_t need = j->dxs.empty() ? fwd : grad;
+    if (need > s->budget) {
+      ome_plan_min_bytes(j->plan, &fwd, &grad);
+      need = j->dxs.empty() ? fwd : grad;
+    }
     if (need > s->budget) {
       s->queue.pop_front();
       reject(s, j, OME_JOB_REJECTED_MEMORY);

@@ -73,6 +73,8 @@ class Plan:
         check(_lib.load().ome_plan_peak_bytes(h, C.byref(fb), C.byref(gb)))
         self.forward_bytes = fb.value
         self.grad_bytes = gb.value
+        check(_lib.load().ome_plan_min_bytes(h, C.byref(fb), C.byref(gb)))
+        self.forward_min, self.grad_min = fb.value, gb.value
         self.ome_dtype = ome_dtype
 
     def __del__(self):

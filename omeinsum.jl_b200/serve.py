@@ -10,7 +10,7 @@ arrival order when a slot is free and the job's planned peak workspace bytes
 (``ome_plan_peak_bytes``) fit a slot's share; a job larger than a share but
 within the whole budget (a gradient job keeps every intermediate) waits until
 the device is idle and runs alone in a workspace of its own size; only jobs
-beyond the budget are rejected.  Work of different jobs overlaps on the
+whose least workspace (``ome_plan_min_bytes``) is beyond the budget are rejected.  Work of different jobs overlaps on the
 device (one stream per slot, the slices of different jobs interleave); a
 finished slot takes the next job at once.  Latency is
 measured from arrival to the completion event of the job's last kernel.
@@ -173,6 +173,8 @@ class TNServer:
             code = code.eins  # gradients run unsliced, as the reference does (src/bp.jl:26-28)
         plan = get_plan(code, sd, p.ome, self.prec)
         need = plan.grad_bytes if job.grad else plan.forward_bytes
+        if need > self.budget:
+            need = plan.grad_min if job.grad else plan.forward_min
         return p, [_f_contig(t) for t in ts], sd, plan, need
 
     def _work(self, job: Job) -> float:

@@ -49,3 +49,30 @@ def test_large_buffers_stay_in_float32():
     p32 = get_plan(tree, size, _lib.F32, 0)
     plain = get_plan(tree, size, _lib.F32, 1)     # (plain Float32: never in Float64)
     assert p32.grad_bytes < 1.2 * plain.grad_bytes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("server", ["TNServer", "NativeTNServer"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_served_within_a_float32_budget(server, grad):
+    """A server whose budget holds the tree's Float32 buffers but not its
+    Float64 ones runs the job (in Float32)."""
+    rng = np.random.default_rng(9)
+    tree, ixs, sd = chain(12, [170], rng)
+    tree = ome.NestedEinsum([tree], ome.EinCode([(0,)], ()))
+    xs = [gen(rng, [170, 170], "f32") / np.float32(np.sqrt(170)) for _ in ixs]
+    plain, full = get_plan(tree, sd, _lib.F32, 1), get_plan(tree, sd, _lib.F32, 0)
+    budget = plain.grad_bytes if grad else plain.forward_bytes
+    assert budget < (full.grad_bytes if grad else full.forward_bytes)
+    srv = getattr(ome, server)(n_slots=1, hbm_budget_bytes=budget)
+    job = ome.Job(tree, [to_dev(x, "f32") for x in xs], grad=grad)
+    st = srv.run_trace([job])
+    srv.close()
+    assert st["completed"] == 1, st
+    ts = [torch.from_numpy(x.astype(np.float64)).requires_grad_() for x in xs]
+    v = torch.diagonal(torch.linalg.multi_dot(ts)).sum()
+    assert_match(to_np(job.value), v.detach().numpy(), "f32")
+    if grad:
+        v.backward()
+        for g, t in zip(job.grads, ts):
+            assert_match(to_np(g), t.grad.numpy(), "f32")
