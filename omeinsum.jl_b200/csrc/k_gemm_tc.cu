@@ -574,8 +574,9 @@ cudaError_t launch_gemm_split(const GemmArgs& g, int nterms, void* workspace, si
 //    running sums in registers (thread = one row x 128 columns) with
 //    round-to-nearest adds.  The cross terms are 2^-8 of the main ones and so is
 //    the round-off of their accumulation: they are drained every fourth chunk.
-//    For the nodes of a sliced tree (GemmArgs::fixed_sums) both are drained
-//    together after 8 stages and joined before the add, as k_gemm_bf16x3 does:
+//    For the nodes of a sliced tree (GemmArgs::fixed_sums) and for more than 512
+//    stages (K > 16384) both are drained together after 8 stages and joined
+//    before the add, as k_gemm_bf16x3 does:
 //    the same time (16384 x 4096 x 4096 and the rest of a sliced 160-vertex
 //    network 15.2 ms either way), error at K = 4097 2.4e-7 instead of 1.7e-7;
 //  * the same warps store the tile (αβ epilogue, or a split partial).
@@ -1274,8 +1275,14 @@ static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, 
   t.S = (int)S;
   t.ksplit = ksplit;
   t.swapped = swapped;
-  t.chunk = g.fixed_sums ? 8 : 4;
-  t.xchunk = g.fixed_sums ? 8 : 16;
+  // Drains every 4 stages truncate less in the accumulator, but add 2.5 times as
+  // often into the running sums, whose rounding grows with the count: from 512
+  // stages on the 8 joined ones are the more exact (K = 16385 2.6e-7 against
+  // 2.7e-7, 32769 3.5e-7 against 3.1e-7, 65537 4.7e-7 against 3.7e-7, at the
+  // same time)
+  const bool joined = g.fixed_sums || (F > 0 ? NKT : ksplit) > 512;
+  t.chunk = joined ? 8 : 4;
+  t.xchunk = joined ? 8 : 16;
   t.units = F + Rt * S;
   const unsigned grid = (unsigned)(2 * std::min<int64_t>(t.units, G));
   // plain launches: a GEMM block started early would hold its SM's shared
