@@ -630,8 +630,7 @@ struct PkArgs {
   int64_t RA, RB;              // 128-row tiles of A and B
   int64_t TM, TN, NKT, tiles, F, ksplit, units;
   int S;
-  int chunk, xchunk;           // stages between two drains of the main and of the cross accumulator (powers of two)
-  int swapped;                 // A and B are the caller's B and A: cross products in the caller's order
+  int swapped;                 // A and B are the caller's B and A: cross products in the caller's order (JOINED)
 };
 
 // One unit of the embedding: 4 consecutive complex k of one row as 8 real
@@ -825,10 +824,13 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
       "h"(mask)
       : "memory");
 }
-template <int NT>
+// JOINED: main and cross accumulators are drained together every 8 stages (an
+// argument in its place costs 2.6% on 1369^3).
+template <int NT, bool JOINED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
     k_gemm_packed(const __grid_constant__ PkArgs t) {
   using namespace pk;
+  constexpr int CHUNK = JOINED ? 8 : 4, XCHUNK = JOINED ? 8 : 16;   // stages between two drains of main and of cross
   constexpr int STAGES = Cfg<NT>::STAGES, STAGE_BYTES = Cfg<NT>::STAGE_BYTES, BLOB = Cfg<NT>::BLOB;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -944,14 +946,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
         decode(u, l, mt, nt, kb, ke, slot);
         const int nk = (int)(ke - kb);
         for (int j = 0; j < nk; ++j, ++it) {
-          const bool first = (j & (t.chunk - 1)) == 0, xfirst = (j & (t.xchunk - 1)) == 0;
+          const bool first = j % CHUNK == 0, xfirst = j % XCHUNK == 0;
           const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
           bool in = true;
           if (xfirst && xc >= 1) in = mbar_wait_cl(xdrained, (xc - 1) & 1, abort_flag);
           in = in && mbar_wait(&full[s], par, abort_flag) && mbar_wait_cl(&peer_full[s], par, abort_flag);
           if (!__all_sync(0xffffffffu, in)) { ok = false; break; }
           tc_fence_after();
-          const bool last = (~j & (t.chunk - 1)) == 0 || j == nk - 1;
+          const bool last = j % CHUNK == CHUNK - 1 || j == nk - 1;
           const uint32_t sa = sbase + s * STAGE_BYTES, sb = sa + BLOB;
           if (elect_one()) {
 #pragma unroll
@@ -961,7 +963,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
               for (int d = 1; d < NT; ++d)
 #pragma unroll
                 for (int i = 0; i <= d; ++i) {
-                  const int ia = t.swapped ? d - i : i;
+                  const int ia = JOINED && t.swapped ? d - i : i;
                   umma_bf16_pair(tmem_cross, umma_desc(sa + ia * TILE_BYTES + kk * 256),
                                  umma_desc(sb + (d - ia) * TILE_BYTES + kk * 256), start ? 0u : 1u, IDESC);
                   start = false;
@@ -984,7 +986,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
           }
           __syncwarp();
           if (last) ++gc;
-          if ((~j & (t.xchunk - 1)) == 0 || j == nk - 1) ++xc;
+          if (j % XCHUNK == XCHUNK - 1 || j == nk - 1) ++xc;
         }
       }
       // every MMA this warp issued must finish before TMEM is freed, and the
@@ -1011,7 +1013,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
     for (int64_t u = cid; u < t.units; u += ncl) {
       int64_t l, mt, nt, kb, ke, slot;
       decode(u, l, mt, nt, kb, ke, slot);
-      const int nch = (int)((ke - kb + t.chunk - 1) / t.chunk);
+      const int nch = (int)((ke - kb + CHUNK - 1) / CHUNK);
       it += (uint32_t)(ke - kb);
       float sum[128];
 #pragma unroll
@@ -1050,11 +1052,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
       for (int ci = 0; ci < nch; ++ci, ++gc) {
         if (!__all_sync(0xffffffffu, mbar_wait_cl(chunk_done, gc & 1, abort_flag))) { ok = false; break; }
         tc_fence_after();
-        if (t.xchunk == t.chunk) {
+        if constexpr (JOINED) {
           drain_pair();
         } else {
           drain(tmem_main, lead_drained);
-          if ((~ci & (t.xchunk / t.chunk - 1)) == 0 || ci == nch - 1) drain(tmem_cross, lead_xdrained);
+          if (ci % (XCHUNK / CHUNK) == XCHUNK / CHUNK - 1 || ci == nch - 1) drain(tmem_cross, lead_xdrained);
         }
       }
       if (!ok) break;
@@ -1189,17 +1191,22 @@ static GemmArgs gemm_swapped(const GemmArgs& q) {
   return g;
 }
 
+template <int NT, bool JOINED>
+static cudaError_t launch_packed_gemm(const PkArgs& t, unsigned grid, cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0};
+  cudaError_t e = set_smem_once(attr, k_gemm_packed<NT, JOINED>, pk::Cfg<NT>::SMEM_BYTES);
+  if (e != cudaSuccess) return e;
+  KernelTimer kt(s, "k_gemm_packed");
+  k_gemm_packed<NT, JOINED><<<grid, pk::NTHREADS, pk::Cfg<NT>::SMEM_BYTES, s>>>(t);
+  count_launch();
+  return cudaGetLastError();
+}
+
 // The packed product of g (its C side, extents in real numbers) whose operands
 // pa and pb describe.
 static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, bool cplx, bool swapped, int nterms,
                                  void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s, int64_t* ctab) {
   using namespace pk;
-  static std::atomic<unsigned long long> attr2{0}, attr3{0};
-  {
-    const cudaError_t e = nterms == 2 ? set_smem_once(attr2, k_gemm_packed<2>, Cfg<2>::SMEM_BYTES)
-                                      : set_smem_once(attr3, k_gemm_packed<3>, Cfg<3>::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-  }
   const int64_t TM = (g.M + BM - 1) / BM, TN = (g.N + BM - 1) / BM, NKT = (g.K + BK - 1) / BK;
   const size_t blob = (size_t)nterms * TILE_BYTES;
   const size_t bytes_a = (size_t)g.L * TM * NKT * blob, bytes_b = (size_t)g.L * TN * NKT * blob;
@@ -1281,19 +1288,12 @@ static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, 
   // 2.7e-7, 32769 3.5e-7 against 3.1e-7, 65537 4.7e-7 against 3.7e-7, at the
   // same time)
   const bool joined = g.fixed_sums || (F > 0 ? NKT : ksplit) > 512;
-  t.chunk = joined ? 8 : 4;
-  t.xchunk = joined ? 8 : 16;
   t.units = F + Rt * S;
   const unsigned grid = (unsigned)(2 * std::min<int64_t>(t.units, G));
   // plain launches: a GEMM block started early would hold its SM's shared
   // memory and TMEM while waiting, which stalls other streams' kernels
-  {
-    KernelTimer kt(s, "k_gemm_packed");
-    if (nterms == 2) k_gemm_packed<2><<<grid, NTHREADS, Cfg<2>::SMEM_BYTES, s>>>(t);
-    else k_gemm_packed<3><<<grid, NTHREADS, Cfg<3>::SMEM_BYTES, s>>>(t);
-  }
-  count_launch();
-  e = cudaGetLastError();
+  if (nterms == 2) e = joined ? launch_packed_gemm<2, true>(t, grid, s) : launch_packed_gemm<2, false>(t, grid, s);
+  else e = joined ? launch_packed_gemm<3, true>(t, grid, s) : launch_packed_gemm<3, false>(t, grid, s);
   if (e != cudaSuccess || Rt == 0) return e;
   k_splitk_tiles<<<(unsigned)std::min<int64_t>(Rt * 64, (int64_t)num_sms * 16), 256, 0, s>>>(t);
   count_launch();
