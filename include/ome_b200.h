@@ -63,7 +63,7 @@ typedef enum {
   OME_TROP_F64 = 7
 } ome_dtype;
 
-/* Precision mode for F32 contractions (other dtypes ignore it).
+/* Precision mode for F32 contractions (other dtypes but C32 ignore it).
  * GEMM-shaped F32 contractions run on the tensor cores as split BF16
  * products accumulated in FP32: each value x = t0 + t1 (+ t2) in bf16.
  * OME_PREC_AUTO   : BF16x6 (3 terms, 6 MMAs per K step; products exact to
@@ -71,7 +71,12 @@ typedef enum {
  * OME_PREC_FP32   : CUDA-core FP32 FMA everywhere (the plain GPU path).
  * OME_PREC_BF16X3 : 2 terms, 3 MMAs (hi*hi + hi*lo + lo*hi); products exact
  *                   to about 2^-16 -- twice as fast, not FP32-accurate.
- * OME_PREC_BF16X6 : same as AUTO. */
+ * OME_PREC_BF16X6 : same as AUTO.
+ * C32 contractions with M, N, K >= 128 and at least 1e9 floating-point
+ * operations run as BF16x6 products of their real parts in every mode but
+ * OME_PREC_FP32, which keeps them on the CUDA cores.  Infinities, NaN and
+ * values outside 2^-60 <= |x| < 2^50 are not split: a product that has any in
+ * its operands is computed on the CUDA cores in every mode. */
 typedef enum { OME_PREC_AUTO = 0, OME_PREC_FP32 = 1, OME_PREC_BF16X3 = 2, OME_PREC_BF16X6 = 3 } ome_prec;
 
 typedef struct {
@@ -129,7 +134,7 @@ OME_API const char* ome_last_error(void);
 /* Create a context on `device` with a device workspace of `workspace_bytes`
  * (intermediates of plans and scratch of single calls).  Replaces the per-
  * intermediate CUDA.jl allocations (ext/CUDAExt.jl:34-47, :129-131).
- * A large FP32 GEMM whose BF16 operand terms do not fit the workspace puts
+ * A large FP32 or ComplexF32 GEMM whose BF16 operand terms do not fit the workspace puts
  * them in a second buffer that the context grows on demand (not during
  * stream capture, at most a quarter of the free device memory; growing
  * synchronises the device) and frees in ome_ctx_destroy. */

@@ -32,10 +32,13 @@ class CuTensorBackend(EinsumBackend):
 class B200Backend(EinsumBackend):
     """The sm_100a backend of this package.
 
-    prec (FP32 only): 0 = AUTO = 3 = BF16X6 (tensor-core products of a 3-term
+    prec (FP32 and large ComplexF32 products): 0 = AUTO = 3 = BF16X6 (tensor-core products of a 3-term
     bf16 split, FP32-faithful), 1 = FP32 (CUDA-core FP32 everywhere, the
     plain GPU path), 2 = BF16X3 (2-term split: twice as fast, about 16-bit
-    products).  Other element types ignore it.
+    products).  ComplexF32 products with M, N, K >= 128 and at least 1e9
+    floating-point operations run as BF16X6 products of their real parts under
+    every value but 1 (on the CUDA cores if an operand holds an infinity, a NaN
+    or a value outside 2^-60 <= |x| < 2^50).  Other element types ignore it.
     """
 
     def __init__(self, prec: int = 0):

@@ -544,6 +544,13 @@ static void* overflow_scratch(ome_ctx* ctx, size_t need, cudaStream_t s) {
   return ctx->ovf;
 }
 
+// A value for RangeFlag::mark that no other launch of this process uses (nor does
+// other data but by a chance of 2^-64).
+static unsigned long long next_mark() {
+  static std::atomic<unsigned long long> count{0};
+  return 0x9e3779b97f4a7c15ull * (count.fetch_add(1, std::memory_order_relaxed) + 1);
+}
+
 static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HView x2, const HView& yu,
                       const Scalar& sx, const Scalar& sy, bool sy_zero, int prec) {
   OME_CK(reduce_dangling(ctx, s, dt, x1, x2, yu));
@@ -702,12 +709,16 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       cudaGetLastError();
     }
     // Large ComplexF32 products on the tensor cores: real BF16x6 products of the
-    // 2 x 2 embedding (1024^3 259 us on the CUDA cores, 77 us here), whose error
-    // of 1.3e-7 .. 2e-7 lies below the CUDA cores' from K = 128 on
+    // 2 x 2 embedding (1024^3 259 us on the CUDA cores, 89 us here), whose error
+    // of 1.2e-7 (K = 128) .. 6.5e-7 (K = 131072) is 0.4 .. 0.07 of the CUDA cores'.
+    // Values that the split cannot hold (infinities, NaN, |x| >= 2^50 or < 2^-60)
+    // are found while the operands are packed: the CUDA-core kernel then computes C
+    // instead (its launch does nothing otherwise; both cost 1024^3 5 us)
     if (dt == OME_C32 && prec != OME_PREC_FP32 && M >= 128 && N >= 128 && K >= 128 && g.sx_one && g.sy_zero &&
         8.0 * (double)M * (double)N * (double)K * (double)L >= 1e9) {
       const size_t top = ctx->ws_top;
       int64_t* tab = static_cast<int64_t*>(ws_alloc(ctx, (size_t)(2 * (M + N)) * sizeof(int64_t)));
+      RangeFlag range = {static_cast<unsigned long long*>(ws_alloc(ctx, sizeof(unsigned long long))), next_mark()};
       size_t avail = ctx->ws_bytes > ctx->ws_top ? ctx->ws_bytes - ((ctx->ws_top + 255) & ~(size_t)255) : 0;
       void* w = avail ? ctx->ws + ((ctx->ws_top + 255) & ~(size_t)255) : nullptr;
       const size_t need = gemm_packed_c32_bytes(g, ctx->num_sms);
@@ -715,10 +726,17 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
         w = overflow_scratch(ctx, need, s);
         avail = w ? ctx->ovf_bytes : 0;
       }
-      const cudaError_t e = tab && w ? launch_gemm_packed_c32(g, w, avail, ctx->num_sms, s, tab) : cudaErrorNotSupported;
+      cudaError_t e = cudaErrorNotSupported;
+      if (tab && range.word && w) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)   // (a graph repeats its mark)
+          OME_CK(cuda_err(cudaMemsetAsync(range.word, 0, sizeof(*range.word), s), "memset"));
+        e = launch_gemm_packed_c32(g, w, avail, ctx->num_sms, s, tab, range);
+      }
       if (e != cudaErrorNotSupported) {
         trace_path("  -> packed complex");
-        return cuda_err(e, "packed complex gemm");
+        OME_CK(cuda_err(e, "packed complex gemm"));
+        return cuda_err(launch_gemm_simt_ws(dt, g, w, avail, ctx->num_sms, s, &range), "simt gemm");
       }
       cudaGetLastError();
       ctx->ws_top = top;

@@ -345,6 +345,15 @@ __host__ __device__ __forceinline__ int64_t mode_offset(int64_t i, int n, const 
   return off;
 }
 
+// A device word that is set to `mark` when an operand holds values that a kernel
+// cannot represent (word NULL: there is no such kernel).  A mark is used once, so
+// that the word needs no reset.
+struct RangeFlag {
+  unsigned long long* word;
+  unsigned long long mark;
+  __device__ bool set() const { return word && *word == mark; }
+};
+
 // Programmatic dependent launch: a kernel launched with the programmatic
 // stream-serialisation attribute (launch_pdl) may start while the previous
 // kernel in its stream finishes; it runs its set-up, then waits in

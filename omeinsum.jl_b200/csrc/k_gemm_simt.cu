@@ -40,6 +40,7 @@ struct SimtArgs {
   int32_t cluster;                 // 1: a tile's splits form a cluster and add up in shared memory
   void* partial;                   // S > 1 without a cluster: [S][L][M][N]
   int64_t p_elems;                 // its capacity in elements (self-check)
+  RangeFlag only_if;               // nothing is done unless this is set (word NULL: always done)
   Scalar sx, sy;
   int sy_zero, sx_one;
 };
@@ -341,6 +342,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_simt(const __grid_const
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
   griddep_launch_dependents();
+  if (g.only_if.word) {
+    griddep_wait();   // the kernels that set it
+    if (!g.only_if.set()) return;
+  }
 
   for (int64_t u = blockIdx.x; u < g.units; u += gridDim.x) {
     int64_t tm, tn, spi, l;
@@ -518,6 +523,7 @@ __global__ void __launch_bounds__(256) k_simt_splitk_finish(const __grid_constan
   constexpr int OUT = 256 / GR;
   __shared__ T part[GR][OUT];
   griddep_wait();   // the partials of the GEMM
+  if (g.only_if.word && !g.only_if.set()) return;
   const T* pp = static_cast<const T*>(g.partial);
   T* Cp = static_cast<T*>(g.C);
   const T sx = scalar_as<T>(g.sx), sy = scalar_as<T>(g.sy);
@@ -636,12 +642,20 @@ static cudaError_t launch_simt_kernel(K* kernel, const SimtArgs& g, int threads,
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)g.S;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
   cfg.attrs = at;
-  cfg.numAttrs = g.cluster ? 1 : 0;
+  cfg.numAttrs = 0;
+  if (g.cluster) {
+    cudaLaunchAttribute& c = at[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeClusterDimension;
+    c.val.clusterDim.x = (unsigned)g.S;
+    c.val.clusterDim.y = c.val.clusterDim.z = 1;
+  }
+  if (g.only_if.word) {   // (it usually returns at once: its launch overlaps the kernel before)
+    cudaLaunchAttribute& c = at[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    c.val.programmaticStreamSerializationAllowed = 1;
+  }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, g);
   count_launch();
   return e;
@@ -966,6 +980,7 @@ static bool simt_args(SimtArgs& g, const GemmArgs& q) {
   g.sy = q.sy;
   g.sy_zero = q.sy_zero;
   g.sx_one = q.sx_one;
+  g.only_if = RangeFlag{nullptr, 0};
   return true;
 }
 
@@ -973,11 +988,12 @@ static bool simt_args(SimtArgs& g, const GemmArgs& q) {
 // partials go to `workspace`.
 template <class A>
 static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, size_t ws_bytes, int num_sms,
-                                         cudaStream_t s) {
+                                         cudaStream_t s, const RangeFlag* only_if) {
   using T = typename A::T;
   if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
   SimtArgs g;
   if (!simt_args(g, q)) return cudaErrorNotSupported;
+  if (only_if) g.only_if = *only_if;
   SimtChoice best;
   if constexpr (std::is_same<A, AlgF64>::value || std::is_same<A, AlgC64>::value) {
     // FP64 matrix instructions once both sides fill a few of their tiles: the
@@ -1227,9 +1243,9 @@ cudaError_t launch_gemm_small_f32(const GemmArgs& q, void* workspace, size_t ws_
 }
 
 cudaError_t launch_gemm_simt_ws(ome_dtype dt, const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms,
-                                cudaStream_t s) {
+                                cudaStream_t s, const RangeFlag* only_if) {
   cudaError_t e = cudaErrorInvalidValue;
-  OME_DISPATCH(dt, ALG, e = launch_gemm_simt_ws_t<ALG>(g, workspace, ws_bytes, num_sms, s));
+  OME_DISPATCH(dt, ALG, e = launch_gemm_simt_ws_t<ALG>(g, workspace, ws_bytes, num_sms, s, only_if));
   return e;
 }
 

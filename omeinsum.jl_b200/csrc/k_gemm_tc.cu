@@ -619,6 +619,7 @@ struct PackArgs {
   // ComplexF32 through its real 2 x 2 embedding: the modes above are complex
   // (R and K count real rows and k), rows of A come in pairs (re, -im), (im, re)
   int a_side;
+  RangeFlag range;    // set if a value is out of the split's range (ComplexF32)
 };
 
 
@@ -631,6 +632,7 @@ struct PkArgs {
   int64_t TM, TN, NKT, tiles, F, ksplit, units;
   int S;
   int swapped;                 // A and B are the caller's B and A: cross products in the caller's order (JOINED)
+  RangeFlag range;             // nothing is done if this is set
 };
 
 // One unit of the embedding: 4 consecutive complex k of one row as 8 real
@@ -658,6 +660,16 @@ __device__ __forceinline__ void load_unit_c32(const float2* __restrict__ base, i
   }
 }
 
+// Whether three BF16 terms of x and the products of its terms stand for x: zero or
+// 2^-60 <= |x| < 2^50.  An infinity or NaN has no finite remainder, a product or
+// sum beyond Float32 would be an infinite main term against an infinite cross
+// term of the other sign, and the accumulators truncate below 2^-126 (512^3 with
+// values about 2^-63 3.6e-7 off, the CUDA cores 2.9e-7, about 2^-60 1.3e-7).
+__device__ __forceinline__ bool in_split_range(float x) {
+  const uint32_t a = __float_as_uint(x) & 0x7fffffffu;
+  return a == 0 || a - ((127u - 60u) << 23) < (110u << 23);
+}
+
 template <int NT, bool CPLX>
 __device__ __forceinline__ void pack_blob(const PackArgs& p, int64_t b, int warp, int lane) {
   using namespace pk;
@@ -683,6 +695,10 @@ __device__ __forceinline__ void pack_blob(const PackArgs& p, int64_t b, int warp
       const int64_t roff = r < p.R ? loff + goff(rc, p.nr, p.r_ext, p.r_str) : -1;
       load_unit_c32(reinterpret_cast<const float2*>(p.X), roff, (kt * BK + kc * 8) >> 1, p.K >> 1, p.kfast, p.nk,
                     p.k_ext, p.k_str, p.a_side ? (int)(r & 1) : 2, v[j]);
+      bool ok = true;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ok = ok && in_split_range(v[j][i]);
+      if (!ok) *p.range.word = p.range.mark;
     } else {
       const int64_t roff = r < p.R ? loff + goff(r, p.nr, p.r_ext, p.r_str) : -1;
       load_unit(p.X, roff, kt * BK + kc * 8, p.K, p.kfast, p.nk, p.k_ext, p.k_str, v[j]);
@@ -832,6 +848,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
   using namespace pk;
   constexpr int CHUNK = JOINED ? 8 : 4, XCHUNK = JOINED ? 8 : 16;   // stages between two drains of main and of cross
   constexpr int STAGES = Cfg<NT>::STAGES, STAGE_BYTES = Cfg<NT>::STAGE_BYTES, BLOB = Cfg<NT>::BLOB;
+  if (t.range.set()) return;   // (the same in both CTAs: an earlier launch has written it)
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* peer_full = full + STAGES;     // (leader) the peer's stage has landed
@@ -1113,6 +1130,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pk::NTHREADS, 1)
 // block takes four columns of a tile, a thread four rows of one (the partials
 // are read as 16-byte vectors, the splits' loads issued together).
 __global__ void __launch_bounds__(256) k_splitk_tiles(const __grid_constant__ PkArgs t) {
+  if (t.range.set()) return;
   const GemmArgs& g = t.g;
   const float sx = scalar_as<float>(g.sx), sy = scalar_as<float>(g.sy);
   float* Cp = static_cast<float*>(g.C);
@@ -1282,6 +1300,7 @@ static cudaError_t launch_packed(const GemmArgs& g, PackArgs& pa, PackArgs& pb, 
   t.S = (int)S;
   t.ksplit = ksplit;
   t.swapped = swapped;
+  t.range = pa.range;
   // Drains every 4 stages truncate less in the accumulator, but add 2.5 times as
   // often into the running sums, whose rounding grows with the count: from 512
   // stages on the 8 joined ones are the more exact (K = 16385 2.6e-7 against
@@ -1345,7 +1364,7 @@ size_t gemm_packed_c32_bytes(const GemmArgs& q, int num_sms) {
 }
 
 cudaError_t launch_gemm_packed_c32(const GemmArgs& q0, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s,
-                                   int64_t* ctab) {
+                                   int64_t* ctab, const RangeFlag& range) {
   const GemmArgs q = q0.n_sc[0] == 1 && q0.m_sc[0] != 1 ? gemm_swapped(q0) : q0;
   GemmArgs g;
   if (!q.sx_one || !q.sy_zero || !c32_embedded(g, q) || !gemm_split_supported(g)) return cudaErrorNotSupported;
@@ -1353,6 +1372,7 @@ cudaError_t launch_gemm_packed_c32(const GemmArgs& q0, void* workspace, size_t w
   pack_args(pa, static_cast<const float*>(q.A), nullptr, g.M, q.nm, q.m_ext, q.m_sa, g, q.k_sa, q.l_sa);
   pack_args(pb, static_cast<const float*>(q.B), nullptr, g.N, q.nn, q.n_ext, q.n_sb, g, q.k_sb, q.l_sb);
   pa.a_side = 1;
+  pa.range = pb.range = range;
   pa.kfast = q.k_sa[0] == 1 && q.k_ext[0] % 4 == 0;
   pb.kfast = q.k_sb[0] == 1 && q.k_ext[0] % 4 == 0;
   return launch_packed(g, pa, pb, true, false, 3, workspace, ws_bytes, num_sms, s, g.nm > 1 || g.nn > 1 ? ctab : nullptr);

@@ -53,9 +53,9 @@ cudaError_t launch_scale(ome_dtype dt, void* y, int nd, const int64_t* ext, cons
 
 // CUDA-core strided batched GEMM over any algebra; K is split over blocks
 // (partials in `workspace`, summed in split order) when the output tiles alone
-// would leave SMs idle.
+// would leave SMs idle.  only_if: nothing is done unless it is set (NULL: always done).
 cudaError_t launch_gemm_simt_ws(ome_dtype dt, const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms,
-                                cudaStream_t s);
+                                cudaStream_t s, const RangeFlag* only_if = nullptr);
 // Small FP32 GEMMs: products and sums in Float64 on the FP64 matrix
 // instructions, rounded once at the end (once per split of K).
 cudaError_t launch_gemm_small_f32(const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s);
@@ -99,9 +99,11 @@ cudaError_t launch_gemm_packed(const GemmArgs& g, int nterms, void* workspace, s
                                cudaStream_t s, int64_t* ctab);
 size_t gemm_packed_bytes(const GemmArgs& g, int nterms, int num_sms);
 // The same for ComplexF32 through its real 2 x 2 embedding (BF16x6 terms); sx = 1
-// and sy = 0 only.  ctab: 2 max(M, N) + min(M, N) entries, or NULL.
+// and sy = 0 only.  ctab: 2 max(M, N) + min(M, N) entries, or NULL.  `range` is
+// set, and C left as it is, if an operand holds a value out of the split's range:
+// an infinity, a NaN, or a nonzero one that is not in 2^-60 <= |x| < 2^50.
 cudaError_t launch_gemm_packed_c32(const GemmArgs& g, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s,
-                                   int64_t* ctab);
+                                   int64_t* ctab, const RangeFlag& range);
 size_t gemm_packed_c32_bytes(const GemmArgs& g, int num_sms);
 // 2-SM tensor-core GEMM fed by TMA tensor maps over the FP32 operands (BF16
 // terms formed in shared memory): single-mode M, N, K and batch groups, each

@@ -23,3 +23,83 @@ def test_long_k_running_sums():
     assert "k_gemm_packed" in names, names
     w = a.double() @ b.double()
     assert float((y.double() - w).norm() / w.norm()) < 4.1e-7
+
+
+def c32(*shape, g):
+    return torch.randn(*shape, dtype=torch.complex64, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("code,shapes", [
+    ("acbd,cedf->eabf", [(9, 13, 33, 21), (13, 10, 21, 170)]),   # two modes in every group, none contiguous in two tensors
+    ("lij,ljk->ikl", [(6, 300, 260), (6, 260, 290)]),            # a batch mode, contiguous in C
+    ("ij,jk->ki", [(257, 1004), (1004, 600)]),                   # K in units of 4, rows on 8 bytes, roles exchanged
+    ("ji,jk->ik", [(1005, 384), (1005, 384)]),                   # a last unit of one k
+])
+@pytest.mark.parametrize("prec", [0, 2])
+def test_c32(code, shapes, prec):
+    """ComplexF32 through the real embedding, on views that start on 8 bytes:
+    norm-wise below 3e-7 (BF16x6 products in FP32 accumulators of 128 real k)."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    xs = [c32(*s[:-1], s[-1] + 1, g=g)[..., 1:] for s in shapes]
+    w = torch.einsum(code, *[x.to(torch.complex128) for x in xs])
+    ome.set_einsum_backend(ome.B200Backend(prec=prec))
+    try:
+        y, names = kernel_names(lambda: ome.ein(code)(*xs))
+    finally:
+        ome.set_einsum_backend(ome.B200Backend())
+    assert "k_gemm_packed" in names, names
+    assert float((y.to(w.dtype) - w).norm() / w.norm()) < 3e-7
+
+
+@pytest.mark.parametrize("value", ["inf", "-inf", "nan", "3.4e38", "1.2e15", "7e-19", "1e-44"])
+@pytest.mark.parametrize("side,at", [(0, (0, 0)), (0, (511, 511)), (1, (300, 511))])
+def test_c32_out_of_range(value, side, at):
+    """A product with a value that BF16 terms do not hold is the CUDA cores'."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    xs = [c32(512, 512, g=g), c32(512, 512, g=g)]
+    code = ome.ein("ij,jk->ik")
+    before = code(*xs)
+    torch.view_as_real(xs[side])[at + (1,)] = float(value)
+    y = code(*xs)
+    again = code(*xs)
+    ome.set_einsum_backend(ome.B200Backend(prec=1))
+    try:
+        w, names = kernel_names(lambda: code(*xs))
+    finally:
+        ome.set_einsum_backend(ome.B200Backend())
+    assert "k_gemm_packed" not in names, names
+    for v in (y, again):
+        assert torch.equal(torch.nan_to_num(torch.view_as_real(v), nan=123.0), torch.nan_to_num(torch.view_as_real(w), nan=123.0))
+    torch.view_as_real(xs[side])[at + (1,)] = 0
+    after, names = kernel_names(lambda: code(*xs))
+    assert "k_gemm_packed" in names, names
+    rows = (slice(None), slice(0, 300)) if side else (slice(1, 511), slice(None))
+    assert torch.equal(after[rows].isfinite(), before[rows].isfinite())
+
+
+def test_c32_out_of_range_in_a_graph():
+    """A captured product takes the path of each replay's values."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    a, b = c32(512, 512, g=g), c32(512, 512, g=g)
+    code = ome.ein("ij,jk->ik")
+    plain = code(a, b)
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(st):
+        code(a, b)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=st):
+            y = code(a, b)
+    for bad in (False, True, False):
+        keep = a[3, 4].clone()
+        if bad:
+            a[3, 4] = float("inf")
+        graph.replay()
+        torch.cuda.synchronize()
+        if bad:
+            assert bool(torch.view_as_real(y)[3].isinf().any())
+            assert torch.equal(torch.isfinite(y).all(dim=1), torch.arange(512, device="cuda") != 3)
+        else:
+            assert torch.equal(y, plain)
+        a[3, 4] = keep
