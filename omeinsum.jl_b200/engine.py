@@ -139,6 +139,8 @@ class _Prepared:
         for t in raw:
             if t.is_conj():
                 t = t.resolve_conj()
+            if t.is_neg():
+                t = t.resolve_neg()
             if t.dtype != self.dtype:
                 t = t.to(device=dev, dtype=self.dtype, non_blocking=True)
             elif t.device != dev:
@@ -299,7 +301,7 @@ def _run_eincode(ixs, iy, p: _Prepared, y: torch.Tensor, sx, sy, loop_only=False
 def plain_layout(xs):
     """(dtype, device index, [shape, strides, ...]) of CUDA tensors that need no
     preparation: plain torch tensors of one supported dtype on one device.
-    None for anything else (host arrays, mixed dtypes, lazy conjugates)."""
+    None for anything else (host arrays, mixed dtypes, lazy conjugates and negatives)."""
     t0 = xs[0]
     if type(t0) is not torch.Tensor or not t0.is_cuda:
         return None
@@ -308,7 +310,7 @@ def plain_layout(xs):
         return None
     lay = []
     for t in xs:
-        if type(t) is not torch.Tensor or t.dtype is not dt or t.get_device() != dev or t.is_conj():
+        if type(t) is not torch.Tensor or t.dtype is not dt or t.get_device() != dev or t.is_conj() or t.is_neg():
             return None
         lay.append(t.shape)
         lay.append(t.stride())

@@ -321,7 +321,7 @@ def tree_gradient(code, xs, dy=None):
     dyp = None
     if dy is not None:
         dyt = dy.data if isinstance(dy, TropicalTensor) else torch.as_tensor(dy)
-        dyt = _f_contig(dyt.to(device=dev, dtype=p.dtype))
+        dyt = _f_contig(dyt.to(device=dev, dtype=p.dtype).resolve_conj().resolve_neg())
         if tuple(dyt.shape) != tuple(shape):
             raise _lib.DimensionMismatch("dy has the wrong shape")
         dyp = dyt
