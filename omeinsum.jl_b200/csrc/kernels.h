@@ -147,6 +147,9 @@ size_t tiny_wide_size(ome_dtype dt);
 // if it does not fit a TinyNode.
 struct HView;
 bool tiny_node(TinyNode& n, int nin, const HView* xs, const HView& y);
+// Whether launch_tiny can run on the current device (arguments as there); its
+// callers ask before the first launch.
+bool tiny_available(ome_dtype dt, bool plain);
 // Runs nodes[0..n) (level[i] ascending); one launch per 100 nodes.  plain: sums
 // and results in the element type itself, with k_loop_thread's arithmetic (for
 // nodes without TINY_WARP; Float32).

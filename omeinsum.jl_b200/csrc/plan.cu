@@ -747,8 +747,12 @@ size_t off_fwd_of(const PNode& n) { return n.off_fwd; }
 size_t off_keep_of(const PNode& n) { return n.off_keep; }
 
 // The descriptors of a tiny program for the caller's input strides, from the
-// plan's cache or built now (pointers are set per launch).
+// plan's cache or built now (pointers are set per launch).  Not ok: the nodes
+// run one by one, as the strides do not fit or the device cannot place the
+// program's cluster.
 std::shared_ptr<const TinyProgram> tiny_program(ome_plan* p, int which, const Leaves& in) {
+  static const auto unavailable = std::make_shared<const TinyProgram>();
+  if (!tiny_available(p->dt, p->fixed_sums)) return unavailable;
   size_t ns = 0;
   for (auto& l : p->in_labels) ns += l.size();
   {

@@ -5,7 +5,7 @@
 // 3-regular bond-2 network with 100 vertices 91 take at most 2^14
 // multiply-adds, 45 of them 32), and one launch each costs 2-3 us on the
 // device and 5 us on the host for nanoseconds of work.  Here one cluster of
-// eight blocks walks the nodes level by level (src/einsequence.jl:270-287
+// sixteen blocks walks the nodes level by level (src/einsequence.jl:270-287
 // evaluates the same nodes in post-order): the nodes of a level are spread
 // over the cluster's warps, and a cluster barrier orders a level's results
 // before the next level's reads.  The descriptors travel as kernel arguments.
@@ -29,7 +29,7 @@ struct TinyArgs {
   uint32_t items[TINY_LEVELS];       // warp items of each level
   TinyNode nodes[CAP];
 };
-// 100 nodes are 32.4 KB of the 32764 bytes a launch's arguments may have
+// 100 nodes are 30.8 KB of the 32764 bytes a launch's arguments may have
 constexpr int TINY_CAP = 100, TINY_CAP_SMALL = 12;
 static_assert(sizeof(TinyArgs<TINY_CAP>) <= 32764, "kernel arguments");
 
@@ -182,6 +182,41 @@ __global__ void __launch_bounds__(TINY_THREADS, 1) k_tiny(const __grid_constant_
   }
 }
 
+// Launch configuration; at: one attribute, filled here.
+cudaLaunchConfig_t tiny_config(cudaLaunchAttribute* at, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(TINY_CTAS);
+  cfg.blockDim = dim3(TINY_THREADS);
+  cfg.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = TINY_CTAS;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Whether the current device can place a cluster of sixteen blocks, which has to
+// be asked for (asked once per device and kernel).
+template <class A, class WA, int CAP>
+bool tiny_fits() {
+  static std::atomic<unsigned long long> asked{0}, fits{0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(asked.load(std::memory_order_acquire) & bit)) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = tiny_config(at, nullptr);
+    int n = 0;
+    cudaError_t e = cudaFuncSetAttribute(k_tiny<A, WA, CAP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, k_tiny<A, WA, CAP>, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    else if (n > 0) fits.fetch_or(bit, std::memory_order_relaxed);
+    asked.fetch_or(bit, std::memory_order_release);
+  }
+  return fits.load(std::memory_order_relaxed) & bit;
+}
+
 template <class A, class WA, int CAP>
 cudaError_t launch_tiny_t(const TinyNode* nodes, const int* level, int n, cudaStream_t s) {
   TinyArgs<CAP> a;
@@ -200,33 +235,25 @@ cudaError_t launch_tiny_t(const TinyNode* nodes, const int* level, int n, cudaSt
   }
   a.items[a.nlevels++] = items;
   a.begin[a.nlevels] = (uint16_t)n;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(TINY_CTAS);
-  cfg.blockDim = dim3(TINY_THREADS);
-  cfg.stream = s;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = TINY_CTAS;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  // sixteen blocks to a cluster have to be asked for
-  static std::atomic<unsigned long long> attr{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(attr.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(k_tiny<A, WA, CAP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    attr.fetch_or(bit, std::memory_order_release);
-  }
-  e = cudaLaunchKernelEx(&cfg, k_tiny<A, WA, CAP>, a);
+  const cudaLaunchConfig_t cfg = tiny_config(at, s);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_tiny<A, WA, CAP>, a);
   count_launch();
   return e;
 }
 
 }  // namespace
+
+bool tiny_available(ome_dtype dt, bool plain) {
+  bool ok = false;
+  if (plain && dt == OME_F32) {
+    ok = tiny_fits<AlgF32, AlgF32, TINY_CAP_SMALL>() && tiny_fits<AlgF32, AlgF32, TINY_CAP>();
+  } else {
+    OME_DISPATCH(dt, ALG, (ok = tiny_fits<ALG, TinyWide<ALG>::W, TINY_CAP_SMALL>() &&
+                                tiny_fits<ALG, TinyWide<ALG>::W, TINY_CAP>()));
+  }
+  return ok;
+}
 
 size_t tiny_wide_size(ome_dtype dt) {
   size_t r = 0;
