@@ -19,7 +19,8 @@ namespace ome {
 // Launch arguments of k_gemm_simt.  The mode groups carry invariant-divisor
 // constants, so that an offset costs four integer instructions per mode
 // instead of a 64-bit division (`wide`: a group's extent does not fit 31 bits
-// and 64-bit divisions are used).
+// and 64-bit divisions are used: div[i].d and .m are then the low and the high
+// half of the mode's extent).
 struct SimtGroup {
   int32_t n;
   FastDiv div[MAXG];
@@ -59,7 +60,7 @@ __device__ __forceinline__ int64_t simt_off(int64_t i, const SimtGroup& g, const
     }
   } else {
     for (int m = 0; m < g.n; ++m) {
-      const int64_t e = g.div[m].d, q = i / e;
+      const int64_t e = (int64_t)(g.div[m].d | (uint64_t)g.div[m].m << 32), q = i / e;
       off += (i - q * e) * str[m];
       i = q;
     }
@@ -936,22 +937,19 @@ static cudaError_t launch_dmma_cfg(SimtArgs& g, const SimtChoice& ch, void* work
   return e != cudaSuccess || g.S == 1 || g.cluster ? e : launch_simt_finish<A>(g, num_sms, s);
 }
 
-static void simt_group(SimtGroup& o, int n, const int64_t* ext, const int64_t* s0, const int64_t* s1) {
+static void simt_group(SimtGroup& o, int n, const int64_t* ext, const int64_t* s0, const int64_t* s1, int wide) {
   o.n = n;
   for (int i = 0; i < n; ++i) {
-    o.div[i] = make_fastdiv((uint32_t)ext[i]);
+    o.div[i] = wide ? FastDiv{(uint32_t)ext[i], (uint32_t)(ext[i] >> 32), 0} : make_fastdiv((uint32_t)ext[i]);
     o.s0[i] = s0[i];
     o.s1[i] = s1[i];
   }
 }
 
-// k_gemm_simt's / k_gemm_dmma's arguments from a contraction; false if an
-// extent does not fit the tables.
-static bool simt_args(SimtArgs& g, const GemmArgs& q) {
-  for (int i = 0; i < q.nm; ++i) if (q.m_ext[i] > 0xffffffffll) return false;
-  for (int i = 0; i < q.nn; ++i) if (q.n_ext[i] > 0xffffffffll) return false;
-  for (int i = 0; i < q.nk; ++i) if (q.k_ext[i] > 0xffffffffll) return false;
-  for (int i = 0; i < q.nl; ++i) if (q.l_ext[i] > 0xffffffffll) return false;
+// k_gemm_simt's / k_gemm_dmma's arguments from a contraction.
+static void simt_args(SimtArgs& g, const GemmArgs& q) {
+  const int64_t lim = (int64_t)1 << 31;
+  g.wide = q.M >= lim || q.N >= lim || q.K >= lim || q.L >= lim;
   g.C = q.C;
   g.K = q.K;
   g.L = q.L;
@@ -960,28 +958,25 @@ static bool simt_args(SimtArgs& g, const GemmArgs& q) {
   const bool swap = q.m_sc[0] == 1 || (q.n_sc[0] != 1 && std::llabs(q.m_sc[0]) < std::llabs(q.n_sc[0]));
   if (!swap) {
     g.A = q.A; g.B = q.B; g.M = q.M; g.N = q.N;
-    simt_group(g.m, q.nm, q.m_ext, q.m_sa, q.m_sc);
-    simt_group(g.n, q.nn, q.n_ext, q.n_sb, q.n_sc);
-    simt_group(g.k, q.nk, q.k_ext, q.k_sa, q.k_sb);
-    simt_group(g.l, q.nl, q.l_ext, q.l_sa, q.l_sb);
+    simt_group(g.m, q.nm, q.m_ext, q.m_sa, q.m_sc, g.wide);
+    simt_group(g.n, q.nn, q.n_ext, q.n_sb, q.n_sc, g.wide);
+    simt_group(g.k, q.nk, q.k_ext, q.k_sa, q.k_sb, g.wide);
+    simt_group(g.l, q.nl, q.l_ext, q.l_sa, q.l_sb, g.wide);
     g.a_rowfast = q.a_m_fast; g.b_rowfast = q.b_n_fast;
   } else {
     g.A = q.B; g.B = q.A; g.M = q.N; g.N = q.M;
-    simt_group(g.m, q.nn, q.n_ext, q.n_sb, q.n_sc);
-    simt_group(g.n, q.nm, q.m_ext, q.m_sa, q.m_sc);
-    simt_group(g.k, q.nk, q.k_ext, q.k_sb, q.k_sa);
-    simt_group(g.l, q.nl, q.l_ext, q.l_sb, q.l_sa);
+    simt_group(g.m, q.nn, q.n_ext, q.n_sb, q.n_sc, g.wide);
+    simt_group(g.n, q.nm, q.m_ext, q.m_sa, q.m_sc, g.wide);
+    simt_group(g.k, q.nk, q.k_ext, q.k_sb, q.k_sa, g.wide);
+    simt_group(g.l, q.nl, q.l_ext, q.l_sb, q.l_sa, g.wide);
     g.a_rowfast = q.b_n_fast; g.b_rowfast = q.a_m_fast;
   }
   for (int i = 0; i < q.nl; ++i) g.l_sc[i] = q.l_sc[i];
-  const int64_t lim = (int64_t)1 << 31;
-  g.wide = g.M >= lim || g.N >= lim || g.K >= lim || g.L >= lim;
   g.sx = q.sx;
   g.sy = q.sy;
   g.sy_zero = q.sy_zero;
   g.sx_one = q.sx_one;
   g.only_if = RangeFlag{nullptr, 0};
-  return true;
 }
 
 // CUDA-core GEMM: tile shape and K split by the estimate above; split
@@ -992,7 +987,7 @@ static cudaError_t launch_gemm_simt_ws_t(const GemmArgs& q, void* workspace, siz
   using T = typename A::T;
   if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
   SimtArgs g;
-  if (!simt_args(g, q)) return cudaErrorNotSupported;
+  simt_args(g, q);
   if (only_if) g.only_if = *only_if;
   SimtChoice best;
   if constexpr (std::is_same<A, AlgF64>::value || std::is_same<A, AlgC64>::value) {
@@ -1232,7 +1227,7 @@ int simt_bounds_flag() {
 cudaError_t launch_gemm_small_f32(const GemmArgs& q, void* workspace, size_t ws_bytes, int num_sms, cudaStream_t s) {
   if (q.M == 0 || q.N == 0 || q.L == 0) return cudaSuccess;
   SimtArgs g;
-  if (!simt_args(g, q)) return cudaErrorNotSupported;
+  simt_args(g, q);
   using E1 = DmmaTile<float, double, 32, 32, 16, 16, 32, 3, 4>;
   using E2 = DmmaTile<float, double, 64, 64, 32, 32, 16, 4, 3>;
   SimtChoice best;

@@ -308,9 +308,10 @@ def plain_layout(xs):
     dt, dev = t0.dtype, t0.get_device()
     if dt not in _TORCH_TO_OME:
         return None
-    lay = []
+    lay, cplx = [], dt.is_complex
     for t in xs:
-        if type(t) is not torch.Tensor or t.dtype is not dt or t.get_device() != dev or t.is_conj() or t.is_neg():
+        if type(t) is not torch.Tensor or t.dtype is not dt or t.get_device() != dev or t.is_neg() or \
+                (cplx and t.is_conj()):
             return None
         lay.append(t.shape)
         lay.append(t.stride())
