@@ -474,13 +474,9 @@ static int reduce_dangling(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView& xu
   return OME_OK;
 }
 
-// Tensor-core kernel for an FP32 GEMM: 2 = the 2-SM kernel fed by tensor
-// maps over the FP32 operands (k_gemm_tma2), 1 = pre-split operands +
-// bulk-copy persistent kernel (k_gemm_packed), 0 = in-kernel converters
-// (k_gemm_bf16x3).  The environment variable OME_GEMM=tma|packed|fused
-// overrides the shape rule (a kernel whose preconditions fail falls through
-// to the next).
-static int gemm_kernel_choice(const GemmArgs& g) {
+// The kernel that the environment variable OME_GEMM=tma|packed|fused asks for
+// (numbers as in gemm_kernel_choice), -1 without it.
+static int gemm_forced() {
   static const int forced = [] {
     const char* e = getenv("OME_GEMM");
     if (!e) return -1;
@@ -489,7 +485,16 @@ static int gemm_kernel_choice(const GemmArgs& g) {
     if (!strcmp(e, "fused")) return 0;
     return -1;
   }();
-  if (forced >= 0) return forced;
+  return forced;
+}
+
+// Tensor-core kernel for an FP32 GEMM: 2 = the 2-SM kernel fed by tensor
+// maps over the FP32 operands (k_gemm_tma2), 1 = pre-split operands +
+// bulk-copy persistent kernel (k_gemm_packed), 0 = in-kernel converters
+// (k_gemm_bf16x3).  OME_GEMM overrides the shape rules, run_binary's too (a
+// kernel whose preconditions fail falls through to the next).
+static int gemm_kernel_choice(const GemmArgs& g) {
+  if (gemm_forced() >= 0) return gemm_forced();
   const double flops = 2.0 * (double)g.M * (double)g.N * (double)g.K * (double)g.L;
   // 256 x 256 cluster tiles: worth it once a few waves of k-steps are there
   if (gemm_tma2_applies(g) && g.M >= 128 && g.N >= 128 && g.K >= 256 && flops >= 2e8) return 2;
@@ -660,7 +665,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       const double macs = (double)M * (double)N * (double)K * (double)L;
       const bool k_scattered =
           g.nk > 1 && (g.k_ext[0] % 8 != 0 || g.k_sa[0] != 1 || g.k_sb[0] != 1);
-      if (choice == 0 && !g.fixed_sums && macs <= (k_scattered ? 0x1p28 : 0x1p25)) {
+      if (choice == 0 && gemm_forced() < 0 && !g.fixed_sums && macs <= (k_scattered ? 0x1p28 : 0x1p25)) {
         trace_path("  -> small");
         cudaError_t e = launch_gemm_small_f32(g, w, avail, ctx->num_sms, s);
         if (e != cudaErrorNotSupported) return cuda_err(e, "small gemm");
@@ -680,7 +685,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       // operands (its products run 1.3 times faster than beside converters):
       // 4096^3 675 -> 600 us, 3072^3 281 -> 269; 2304^3 130 against 138,
       // 8192 x 512 x 8192 358 against 431
-      const bool prefer_packed = choice == 2 && !g.fixed_sums && K >= 2048 && M * N >= 1536 * (M + N) &&
+      const bool prefer_packed = choice == 2 && gemm_forced() < 0 && !g.fixed_sums && K >= 2048 && M * N >= 1536 * (M + N) &&
                                  gemm_packed_bytes(g, nterms, ctx->num_sms) <= avail;
       if (choice == 1 || prefer_packed) {
         cudaError_t e = packed();
@@ -692,13 +697,15 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       }
       if (choice == 2) {
         cudaError_t e = launch_gemm_tma2(g, nterms, w, avail, ctx->num_sms, s);
-        if (e == cudaErrorNotSupported) {
-          cudaGetLastError();
-          e = packed();
-        }
         if (e != cudaErrorNotSupported) {
           trace_path("  -> tma2");
           return cuda_err(e, "tma bf16 split gemm");
+        }
+        cudaGetLastError();
+        e = packed();
+        if (e != cudaErrorNotSupported) {
+          trace_path("  -> packed");
+          return cuda_err(e, "packed bf16 split gemm");
         }
         cudaGetLastError();
       }

@@ -1,5 +1,9 @@
 """The packed tensor-core GEMM (k_gemm_packed): rows on 4-byte boundaries, so
 that no tensor map describes the operands."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -103,3 +107,32 @@ def test_c32_out_of_range_in_a_graph():
         else:
             assert torch.equal(y, plain)
         a[3, 4] = keep
+
+
+FORCED = """
+import sys; sys.path[:0] = ["tests", "oracle", "."]
+import conftest, torch
+import omeinsum_b200 as ome
+from test_gpu_parity import kernel_names
+for m, n, k in ((3072, 3072, 2048), (64, 64, 64)):
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    y, names = kernel_names(lambda: ome.ein("ij,jk->ik")(a, b))
+    assert float((y - a.double() @ b.double()).norm() / y.norm()) < 1e-6
+    print(*names)
+"""
+
+
+@pytest.mark.parametrize("kernel,names", [
+    ("", ["k_gemm_packed", "k_gemm_dmma"]),
+    ("tma", ["k_gemm_tma2", "k_gemm_tma2"]),
+    ("packed", ["k_gemm_packed", "k_gemm_packed"]),
+    ("fused", ["k_gemm_bf16x3", "k_gemm_bf16x3"]),
+])
+def test_kernel_of_choice(kernel, names):
+    """OME_GEMM selects the kernel whatever the size."""
+    env = dict(os.environ, OME_GEMM=kernel)
+    r = subprocess.run([sys.executable, "-c", FORCED], env=env, capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
+    got = [line.split()[-1] for line in r.stdout.split("\n") if line.startswith("k_")]
+    assert got == names, r.stdout
