@@ -656,7 +656,7 @@ static int run_binary(ome_ctx* ctx, cudaStream_t s, ome_dtype dt, HView x1, HVie
       // Small products on the FP64 matrix instructions: below 2^25 multiply-adds
       // the tensor-core kernel's fixed 11-25 us (two operands' splits, eight
       // k-steps of accumulators) exceed the whole product here (64 x 16 x 8
-      // 10.6 -> 5.8 us, 256^3 24.4 -> 12.3, 512 x 512 x 128 17.7 -> 12.3; above,
+      // 9.7 -> 5.1 us, 256^3 22.6 -> 9.2, 512 x 512 x 128 17.1 -> 13.0; above,
       // 1024 x 1024 x 64 13.9 against 19.6), and sums in Float64 are the more
       // exact.  Where an operand's K runs over several modes and is not
       // contiguous, its converters evaluate a mixed-radix offset per element and

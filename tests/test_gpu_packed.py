@@ -29,6 +29,50 @@ def test_long_k_running_sums():
     assert float((y.double() - w).norm() / w.norm()) < 4.1e-7
 
 
+@pytest.mark.parametrize("code,shapes", [
+    ("ij,jk->ki", [(641, 1030), (1030, 1150)]),                        # 6 and 9 tiles of 128: an odd one on the second side
+    ("ij,jk->ik", [(1150, 1030), (1030, 641)]),                        # the same with the operands' roles exchanged
+    ("acbd,cedf->eabf", [(11, 33, 61, 23), (33, 20, 23, 55)]),         # two modes that do not merge in every group
+    ("lij,ljk->lki", [(3, 390, 517), (3, 517, 970)]),                  # a batch mode
+    ("ij,jk->ik", [(2050, 600), (600, 2900)]),                         # 9 x 12 tiles of 256: whole tiles and split ones
+])
+@pytest.mark.parametrize("prec", [0, 2, 3])
+def test_f32(code, shapes, prec):
+    """Float32 on rows that start on 4 bytes, with y <- 3 f + 2 y.  Norm-wise:
+    three terms 3e-7 (FP32 accumulators of 128 to 256 k), two terms 1e-5 (a
+    value's two terms leave 2^-17 of it)."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    xs = [torch.randn(*s[:-1], s[-1] + 1, generator=g, device="cuda")[..., 1:] for s in shapes]
+    w = torch.einsum(code, *[x.double() for x in xs])
+    tol = 1e-5 if prec == 2 else 3e-7
+    ome.set_einsum_backend(ome.B200Backend(prec=prec))
+    try:
+        y, names = kernel_names(lambda: ome.ein(code)(*xs))
+        assert "k_gemm_packed" in names, names
+        assert float((y - w).norm() / w.norm()) < tol
+        for out in (torch.randn(w.shape, generator=g, device="cuda"),
+                    torch.randn(w.shape[::-1], generator=g, device="cuda").permute(*range(w.dim() - 1, -1, -1))):
+            want = 3 * w + 2 * out.double()
+            _, names = kernel_names(lambda: ome.einsum_(ome.ein(code), xs, out, 3, 2))
+            assert "k_gemm_packed" in names, names
+            assert float((out - want).norm() / want.norm()) < tol
+    finally:
+        ome.set_einsum_backend(ome.B200Backend())
+
+
+@pytest.mark.parametrize("m,n,k", [(3072, 3072, 2048), (2304, 5000, 2304)])
+def test_f32_aligned(m, n, k):
+    """Large square-ish products take the packed kernel although tensor maps
+    describe their operands."""
+    g = torch.Generator(device="cuda").manual_seed(10)
+    a, b = torch.randn(m, k, generator=g, device="cuda"), torch.randn(k, n, generator=g, device="cuda")
+    w = a.double() @ b.double()
+    for code in ("ij,jk->ik", "ij,jk->ki"):
+        y, names = kernel_names(lambda: ome.ein(code)(a, b))
+        assert names[0] == "k_gemm_packed", names
+        assert float(((y if code[-1] == "k" else y.t()) - w).norm() / w.norm()) < 3e-7
+
+
 def c32(*shape, g):
     return torch.randn(*shape, dtype=torch.complex64, generator=g, device="cuda")
 
