@@ -175,6 +175,7 @@ class Context:
     def __init__(self, device: int, workspace_bytes: int):
         self.device = device
         self.workspace_bytes = int(workspace_bytes)
+        self.refused: float = float("inf")   # a larger workspace that the device did not have
         h = C.c_void_p()
         check(load().ome_ctx_create(device, self.workspace_bytes, C.byref(h)))
         self.handle = h
@@ -205,17 +206,36 @@ def release_workspaces() -> None:
 DEFAULT_WORKSPACE = 256 << 20
 
 
-def context(device: int, min_workspace: int = 0) -> Context:
+def context(device: int, min_workspace: int = 0, least: int | None = None) -> Context:
     """The context of `device`, grown (re-created) if its workspace is smaller
-    than `min_workspace` bytes."""
+    than `min_workspace` bytes.  If the device does not have that much memory,
+    `least` bytes (where given) will do."""
     import torch
 
     c = _contexts.get(device)
+    if c is not None and c.workspace_bytes >= min_workspace:
+        return c
+    if least is None:
+        least = min_workspace
+    if c is not None and c.workspace_bytes >= least and min_workspace >= c.refused:
+        return c
     need = max(min_workspace, DEFAULT_WORKSPACE)
-    if c is None or c.workspace_bytes < min_workspace:
-        if c is not None:
-            torch.cuda.synchronize(device)
-            c.close()
-        c = Context(device, need if c is None else max(need, c.workspace_bytes * 2, min_workspace))
+    old = 0
+    if c is not None:
+        old = c.workspace_bytes
+        torch.cuda.synchronize(device)
+        del _contexts[device]
+        c.close()
+    sizes = sorted({max(need, 2 * old), need, max(least, min(old, need), DEFAULT_WORKSPACE), least}, reverse=True)
+    for size in sizes:
+        try:
+            c = Context(device, size)
+        except MemoryError:
+            if size == sizes[-1]:
+                raise
+            continue
+        if size < min_workspace:
+            c.refused = min_workspace
         _contexts[device] = c
-    return c
+        return c
+    raise AssertionError("unreachable")

@@ -127,7 +127,7 @@ class ShardedSlices:
             raise ArgumentError("inputs changed element type since planning")
         ins = [_f_contig(t) for t in p.tensors]
         part = _alloc(self.out_shape, self.partial_dtype, self.device)
-        ctx = _lib.context(self.device.index, self.plan.forward_bytes)
+        ctx = _lib.context(self.device.index, self.plan.forward_bytes, self.plan.forward_min)
         b, e = self.range
         with torch.cuda.device(self.device):
             check(_lib.load().ome_plan_execute_slices(ctx.handle, self.plan.handle, _stream(self.device), _ptrs(ins),
@@ -142,7 +142,7 @@ class ShardedSlices:
         yt = _alloc(self.out_shape, self.dtype, self.device) if y is None else y
         if tuple(yt.shape) != tuple(self.out_shape) or tuple(yt.stride()) != tuple(_f_contig(yt).stride()):
             raise ArgumentError("y must be a column-major array of the output shape")
-        ctx = _lib.context(self.device.index, self.plan.forward_bytes)
+        ctx = _lib.context(self.device.index, self.plan.forward_bytes, self.plan.forward_min)
         with torch.cuda.device(self.device):
             check(_lib.load().ome_plan_finish(ctx.handle, self.plan.handle, _stream(self.device), part.data_ptr(),
                                               yt.data_ptr(), _scalar_buf(self.ome, sx), _scalar_buf(self.ome, sy)))

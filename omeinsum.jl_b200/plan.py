@@ -256,7 +256,7 @@ def tree_plain(code, xs):
         return None
     call, trop, raw = got
     raw, ptrs = call.prepare(raw)
-    ctx = _lib.context(call.dev, call.plan.forward_bytes)
+    ctx = _lib.context(call.dev, call.plan.forward_bytes, call.plan.forward_min)
     y = torch.empty_strided(call.shape, call.strides, dtype=call.dtype, device=call.device)
     check(_lib.load().ome_plan_execute_strided(ctx.handle, call.plan.handle, _raw_stream(call.dev), ptrs, call.str,
                                                y.data_ptr(), call.one, call.zero))
@@ -273,7 +273,7 @@ def gradient_plain(code, xs):
         return None
     call, trop, raw = got
     raw, ptrs = call.prepare(raw)
-    ctx = _lib.context(call.dev, call.plan.grad_bytes)
+    ctx = _lib.context(call.dev, call.plan.grad_bytes, call.plan.grad_min)
     y = torch.empty_strided(call.shape, call.strides, dtype=call.dtype, device=call.device)
     new, dt, dev = torch.empty_strided, call.dtype, call.device
     dxs = [new(sh, st, dtype=dt, device=dev) for sh, st in call.xlay]
@@ -302,7 +302,7 @@ def run_tree(code, xs, size_dict=None, y=None, sx=True, sy=False):
     p = _Prepared(xs, out_dtype=out_dtype)
     plan = get_plan(code, size_dict, p.ome, be.prec)
     dev = p.device
-    ctx = _lib.context(dev.index, plan.forward_bytes)
+    ctx = _lib.context(dev.index, plan.forward_bytes, plan.forward_min)
     ins = [_f_contig(t) for t in p.tensors]
     shape = [size_dict[l] for l in ne.eins.iy]
     if y is None:
@@ -340,7 +340,7 @@ def tree_gradient(code, xs, dy=None):
     p = _Prepared(xs)
     plan = get_plan(ne, size_dict, p.ome, be.prec)
     dev = p.device
-    ctx = _lib.context(dev.index, plan.grad_bytes)
+    ctx = _lib.context(dev.index, plan.grad_bytes, plan.grad_min)
     ins = [_f_contig(t) for t in p.tensors]
     shape = [size_dict[l] for l in ne.eins.iy]
     yt = _alloc(shape, p.dtype, dev)
