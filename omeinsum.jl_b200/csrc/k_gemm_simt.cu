@@ -733,8 +733,9 @@ __device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[2], doubl
 // shared-memory wavefronts per multiply-add are a third of k_gemm_simt's,
 // which bound that one.  Float64 1681^3 (rows on 8-byte boundaries) 1200 ->
 // 450 us, 21 TFLOP/s; 2368 x 2048 x 2048 25 TFLOP/s of the pipe's 37; the
-// matrix pipe is 71% busy, the rest is the fixed wait between dependent issues
-// with at most 12 warps on an SM.
+// matrix pipe is 64% busy over the 1.6 waves of 1681^3, the rest is their last
+// part and the fixed wait between dependent issues with at most 12 warps on an
+// SM.
 template <class A, class C>
 __global__ void __launch_bounds__(C::NT, C::MINB) k_gemm_dmma(const __grid_constant__ SimtArgs g) {
   using T = typename A::T;
