@@ -12,7 +12,7 @@
     B200Backend(; prec = 0)
 
 Einsum on NVIDIA B200 GPUs through `libomeb200` (hand-written sm_100a
-kernels).  `prec` selects how Float32 contractions use the tensor cores:
+kernels).  `prec` selects how Float32 (and large ComplexF32) contractions use the tensor cores:
 0 = automatic (BF16x6 split products, FP32-faithful), 1 = plain FP32 on CUDA
 cores, 2 = BF16x3, 3 = BF16x6.  Other element types (Float64, complex,
 Int64, Bool, Tropical) are exact on CUDA cores.  With this backend selected,
