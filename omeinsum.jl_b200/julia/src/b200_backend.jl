@@ -14,9 +14,11 @@
 Einsum on NVIDIA B200 GPUs through `libomeb200` (hand-written sm_100a
 kernels).  `prec` selects how Float32 (and large ComplexF32) contractions use the tensor cores:
 0 = automatic (BF16x6 split products, FP32-faithful), 1 = plain FP32 on CUDA
-cores, 2 = BF16x3, 3 = BF16x6.  Other element types (Float64, complex,
-Int64, Bool, Tropical) are exact on CUDA cores.  With this backend selected,
-an unsupported case is an error, never a CPU fallback.
+cores, 2 = BF16x3, 3 = BF16x6; ComplexF32 products with M, N, K >= 128 and at
+least 1e9 operations are BF16x6 under every value but 1.  Other element types
+(Float64, ComplexF64, Int64, Bool, Tropical) are computed in their own
+arithmetic whatever the value.  With this backend selected, an unsupported case
+is an error, never a CPU fallback.
 """
 struct B200Backend <: EinsumBackend
     prec::Int32
